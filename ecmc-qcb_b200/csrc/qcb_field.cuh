@@ -303,7 +303,7 @@ struct AlgField {
         const int nT = (int)((Vh + 31) >> 5);
         return (size_t)((mu * 2 + par) * nT + (h >> 5)) * (4 * 32);
     }
-    __device__ __forceinline__ M3<R> load(int mu, int par, int h) const {
+    __device__ __forceinline__ AntiH<R> load(int mu, int par, int h) const {
         C2 z01, z02, z12, dg;
         if constexpr (kQuad) {
             const float4* q = reinterpret_cast<const float4*>(p + tile0(mu, par, h)) + (h & 31);
@@ -319,37 +319,34 @@ struct AlgField {
             z12 = b[64];
             dg = b[96];
         }
-        M3<R> z;
-        z(0, 1) = mkc<R>(z01.x, z01.y);
-        z(0, 2) = mkc<R>(z02.x, z02.y);
-        z(1, 2) = mkc<R>(z12.x, z12.y);
-        z(1, 0) = mkc<R>(-z01.x, z01.y);
-        z(2, 0) = mkc<R>(-z02.x, z02.y);
-        z(2, 1) = mkc<R>(-z12.x, z12.y);
-        z(0, 0) = mkc<R>(0, dg.x);
-        z(1, 1) = mkc<R>(0, dg.y);
-        z(2, 2) = mkc<R>(0, -(dg.x + dg.y));
+        AntiH<R> z;
+        z.o[0] = mkc<R>(z01.x, z01.y);
+        z.o[1] = mkc<R>(z02.x, z02.y);
+        z.o[2] = mkc<R>(z12.x, z12.y);
+        z.d[0] = dg.x;
+        z.d[1] = dg.y;
+        z.d[2] = -(dg.x + dg.y);
         return z;
     }
-    __device__ __forceinline__ void store(int mu, int par, int h, const M3<R>& z) const {
+    __device__ __forceinline__ void store(int mu, int par, int h, const AntiH<R>& z) const {
         if constexpr (kQuad) {
             float4* q = reinterpret_cast<float4*>(p + tile0(mu, par, h)) + (h & 31);
-            q[0] = make_float4(z(0, 1).re, z(0, 1).im, z(0, 2).re, z(0, 2).im);
-            q[32] = make_float4(z(1, 2).re, z(1, 2).im, z(0, 0).im, z(1, 1).im);
+            q[0] = make_float4(z.o[0].re, z.o[0].im, z.o[1].re, z.o[1].im);
+            q[32] = make_float4(z.o[2].re, z.o[2].im, z.d[0], z.d[1]);
         } else {
             C2* b = p + tile0(mu, par, h) + (h & 31);
             C2 v;
-            v.x = z(0, 1).re;
-            v.y = z(0, 1).im;
+            v.x = z.o[0].re;
+            v.y = z.o[0].im;
             b[0] = v;
-            v.x = z(0, 2).re;
-            v.y = z(0, 2).im;
+            v.x = z.o[1].re;
+            v.y = z.o[1].im;
             b[32] = v;
-            v.x = z(1, 2).re;
-            v.y = z(1, 2).im;
+            v.x = z.o[2].re;
+            v.y = z.o[2].im;
             b[64] = v;
-            v.x = z(0, 0).im;
-            v.y = z(1, 1).im;
+            v.x = z.d[0];
+            v.y = z.d[1];
             b[96] = v;
         }
     }

@@ -108,27 +108,27 @@ struct FmtImpl {
     }
     static cudaError_t flow1(const Geom& g, const void* win, void* wout, void* z, double eps, int stage, int rep,
                              cudaStream_t s) {
-        const unsigned nb = 8u * (unsigned)((g.Vh + QCB_FLOW1_THREADS - 1) / QCB_FLOW1_THREADS);
+        const unsigned nb = 8u * (unsigned)((g.Vh + QCB_FLOW_THREADS - 1) / QCB_FLOW_THREADS);
         AlgField<R> za;
         za.p = (typename AlgField<R>::C2*)z;
         za.Vh = g.Vh;
         if (stage == 1)
-            k_flow_stage<R, NE, 1><<<nb, QCB_FLOW1_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps, rep);
+            k_flow_stage<R, NE, 1><<<nb, QCB_FLOW_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps, rep);
         else if (stage == 2)
-            k_flow_stage<R, NE, 2><<<nb, QCB_FLOW1_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps, rep);
+            k_flow_stage<R, NE, 2><<<nb, QCB_FLOW_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps, rep);
         else
-            k_flow_stage<R, NE, 3><<<nb, QCB_FLOW1_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps, rep);
+            k_flow_stage<R, NE, 3><<<nb, QCB_FLOW_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps, rep);
         return cudaGetLastError();
     }
 
     static cudaError_t flow1_meas(const Geom& g, const void* win, void* wout, void* z, double eps, int rep,
                                   void* hbuf, cudaStream_t s) {
-        const unsigned nb = 8u * (unsigned)((g.Vh + QCB_FLOW1_THREADS - 1) / QCB_FLOW1_THREADS);
+        const unsigned nb = 8u * (unsigned)((g.Vh + QCB_FLOW_THREADS - 1) / QCB_FLOW_THREADS);
         AlgField<R> za;
         za.p = (typename AlgField<R>::C2*)z;
         za.Vh = g.Vh;
         const HalfClovers<R> H{(R*)hbuf, 2 * g.Vh};
-        k_flow_stage1_meas<R, NE><<<nb, QCB_FLOW1_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps,
+        k_flow_stage1_meas<R, NE><<<nb, QCB_FLOW_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps,
                                                                    rep, H);
         return cudaGetLastError();
     }
@@ -145,8 +145,8 @@ struct FmtImpl {
         return z;
     }
     static cudaError_t flow_force(const Geom& g, const void* w, void* f, cudaStream_t s) {
-        const unsigned nb = 8u * (unsigned)((g.Vh + QCB_FLOW1_THREADS - 1) / QCB_FLOW1_THREADS);
-        k_flow_force<R, NE><<<nb, QCB_FLOW1_THREADS, 0, s>>>(g, view(w, g.Vh), alg(f, g.Vh));
+        const unsigned nb = 8u * (unsigned)((g.Vh + QCB_FLOW_THREADS - 1) / QCB_FLOW_THREADS);
+        k_flow_force<R, NE><<<nb, QCB_FLOW_THREADS, 0, s>>>(g, view(w, g.Vh), alg(f, g.Vh));
         return cudaGetLastError();
     }
     static cudaError_t flow_update(const Geom& g, void* w, const void* f0, const void* f1, double a, double b,

@@ -135,7 +135,9 @@ __device__ __forceinline__ M3<R> staple_rt(const Geom& g, const LinkField<R, NE>
 // rows 0-1 of t^dag need columns 0-1 of t only.  That is 42 instead of 54 complex
 // multiply-adds a staple.  The rebuilt row differs from the explicit product by the
 // links' distance from SU(3), which in FP32 storage is the FP32 rounding level (~1e-7).
-template <typename R, int NE>
+// FLOW: the flow kernels' order of nu, mu ^ 1, mu ^ 2, mu ^ 3, in which the warps of mu and nu are in the
+// same plane at the same time and share its links in L1; else ascending, as compute_staple.
+template <typename R, int NE, bool FLOW = false>
 __device__ __forceinline__ M3<R> staple_rt_rows(const Geom& g, const LinkField<R, NE>& U, const int c[4],
                                                 int lex, int par, int mu) {
     M3<R> A;
@@ -145,7 +147,7 @@ __device__ __forceinline__ M3<R> staple_rt_rows(const Geom& g, const LinkField<R
     const int xmu = lex + sel4(st.up, mu);
 #pragma unroll 1
     for (int k = 0; k < 3; k++) {
-        const int nu = k < mu ? k : k + 1;
+        const int nu = FLOW ? mu ^ (k + 1) : (k < mu ? k : k + 1);
         const int dnu = sel4(st.dn, nu);
         const int xnu = lex + sel4(st.up, nu);
         const int xmnu = lex + dnu;
@@ -302,7 +304,7 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
     const int64_t site = (int64_t)par * g.Vh + (lex >> 1), site_up = (int64_t)opp * g.Vh + (xmu >> 1);
 #pragma unroll 1
     for (int k = 0; k < 3; k++) {
-        const int nu = k < mu ? k : k + 1;
+        const int nu = mu ^ (k + 1);
         const int plane = mu < nu ? plane_index(mu, nu) : plane_index(nu, mu);
         const bool owned = plane_owner(plane) == mu;
         const int dnu = sel4(st.dn, nu);
@@ -399,33 +401,29 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
 // -proj_lie(u A) (compute_force, gradient_flow.cpp:17-37) forming only the entries the
 // projection reads: the six off-diagonal entries of u A and the imaginary parts of its diagonal.
 template <typename R>
-__device__ __forceinline__ M3<R> neg_proj_lie_mul(const M3<R>& u, const M3<R>& A) {
-    M3<R> m;
+__device__ __forceinline__ AntiH<R> neg_proj_lie_mul(const M3<R>& u, const M3<R>& A) {
+    R im[3];
+    AntiH<R> F;
+    const int I[3] = {0, 0, 1}, J[3] = {1, 2, 2};
 #pragma unroll
-    for (int i = 0; i < 3; i++)
+    for (int i = 0; i < 3; i++) {
+        im[i] = R(0);
 #pragma unroll
-        for (int j = 0; j < 3; j++) {
-            if (i == j) {
-                R im = R(0);
+        for (int q = 0; q < 3; q++) im[i] = fma(u(i, q).re, A(q, i).im, fma(u(i, q).im, A(q, i).re, im[i]));
+    }
 #pragma unroll
-                for (int q = 0; q < 3; q++) im = fma(u(i, q).re, A(q, i).im, fma(u(i, q).im, A(q, i).re, im));
-                m(i, i) = mkc<R>(R(0), im);
-            } else {
-                Cx<R> v = mkc<R>(0, 0);
+    for (int k = 0; k < 3; k++) {
+        Cx<R> v = mkc<R>(0, 0), w = mkc<R>(0, 0);
 #pragma unroll
-                for (int q = 0; q < 3; q++) cmac(v, u(i, q), A(q, j));
-                m(i, j) = v;
-            }
+        for (int q = 0; q < 3; q++) {
+            cmac(v, u(I[k], q), A(q, J[k]));
+            cmac(w, u(J[k], q), A(q, I[k]));
         }
-    M3<R> F;
+        F.o[k] = mkc<R>(R(0.5) * (w.re - v.re), R(-0.5) * (v.im + w.im));
+    }
+    const R tr3 = (im[0] + im[1] + im[2]) * R(1.0 / 3.0);
 #pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-            if (i != j) F(i, j) = mkc<R>(R(-0.5) * (m(i, j).re - m(j, i).re), R(-0.5) * (m(i, j).im + m(j, i).im));
-    const R tr3 = (m(0, 0).im + m(1, 1).im + m(2, 2).im) / R(3);
-#pragma unroll
-    for (int i = 0; i < 3; i++) F(i, i) = mkc<R>(R(0), tr3 - m(i, i).im);
+    for (int i = 0; i < 3; i++) F.d[i] = tr3 - im[i];
     return F;
 }
 
@@ -455,10 +453,6 @@ __device__ __forceinline__ M3<R> neg_proj_lie_mul(const M3<R>& u, const M3<R>& A
 #ifndef QCB_CLOVER_MINB
 #define QCB_CLOVER_MINB(R) (sizeof(R) == 8 ? 2 : 4)
 #endif
-// single-lattice flow stage launch shape (the tiled kernels keep QCB_FLOW_THREADS = TILE)
-#ifndef QCB_FLOW1_THREADS
-#define QCB_FLOW1_THREADS QCB_FLOW_THREADS
-#endif
 #ifndef QCB_FLOW1_MINB
 #define QCB_FLOW1_MINB(R) (sizeof(R) == 8 ? 3 : 6)
 #endif
@@ -467,15 +461,9 @@ __device__ __forceinline__ M3<R> neg_proj_lie_mul(const M3<R>& u, const M3<R>& A
 #ifndef QCB_FLOW_MEAS_MINB
 #define QCB_FLOW_MEAS_MINB(R) (sizeof(R) == 8 ? 3 : 4)
 #endif
-#ifndef QCB_FLOW_RTMU
-#define QCB_FLOW_RTMU 1
-#endif
-// FP64 flow stages and clover leaves with two-row products (third row rebuilt as conj(r0 x r1)),
-// as in FP32.  The rebuilt rows differ from explicit products by the links' distance from SU(3),
-// ~1e-15 in FP64, inside the 1e-12 parity bound; the flow stage runs 8% faster.
-#ifndef QCB_FLOW64_ROWS
-#define QCB_FLOW64_ROWS 1
-#endif
+// FP64 clover leaves with two-row products (third row rebuilt as conj(r0 x r1)), as in FP32.  The
+// rebuilt rows differ from explicit products by the links' distance from SU(3), ~1e-15 in FP64,
+// inside the 1e-12 parity bound.
 #ifndef QCB_CLOVER64_ROWS
 #define QCB_CLOVER64_ROWS 1
 #endif
@@ -874,12 +862,12 @@ template <typename R, int NE, int STAGE, bool MEAS = false>
 __device__ __forceinline__ void flow_link(const Geom& g, const LinkField<R, NE>& Win, const LinkField<R, NE>& Wout,
                                           const AlgField<R>& Z, double eps, int mu, int par, int h,
                                           int reproject, const HalfClovers<R>& H = HalfClovers<R>{}) {
-    static_assert(!MEAS || (STAGE == 1 && (sizeof(R) == 4 || QCB_FLOW64_ROWS)),
-                  "the clover halves come from stage 1's two-row staples");
+    static_assert(!MEAS || STAGE == 1, "the clover halves come from stage 1's staples");
     int c[4];
     site_coords(g, par, (uint32_t)h, c);
     const int lex = lex_of(g, c);
-    M3<R> F, u;
+    AntiH<R> F;
+    M3<R> u;
     if constexpr (MEAS) {
         // the same staple and force, with the clover halves of the input configuration
         if constexpr (sizeof(R) == 8) {  // the link reloaded where the halves need it
@@ -891,50 +879,24 @@ __device__ __forceinline__ void flow_link(const Geom& g, const LinkField<R, NE>&
             const M3<R> A = staple_rt_rows_meas<R, NE>(g, Win, c, lex, par, mu, u, H);
             F = neg_proj_lie_mul(u, A);
         }
-    } else if constexpr (sizeof(R) == 4 || QCB_FLOW64_ROWS) {
+    } else {
         // two-row staple products and the projection's entries only
-        const M3<R> A = staple_rt_rows<R, NE>(g, Win, c, lex, par, mu);
+        const M3<R> A = staple_rt_rows<R, NE, true>(g, Win, c, lex, par, mu);
         u = Win.load_ro(mu, par, h);
         F = neg_proj_lie_mul(u, A);
-    } else {
-        M3<R> A;
-#if QCB_FLOW_RTMU
-        A = staple_rt<R, NE>(g, Win, c, lex, par, mu);
-#else
-        switch (mu) {
-            case 0: A = staple<R, NE, 0, true>(g, Win, c, lex, par); break;
-            case 1: A = staple<R, NE, 1, true>(g, Win, c, lex, par); break;
-            case 2: A = staple<R, NE, 2, true>(g, Win, c, lex, par); break;
-            default: A = staple<R, NE, 3, true>(g, Win, c, lex, par); break;
-        }
-#endif
-        u = Win.load_ro(mu, par, h);
-        F = proj_lie(mul_nn(u, A));
-#pragma unroll
-        for (int k = 0; k < 9; k++) F.e[k] = mkc<R>(-F.e[k].re, -F.e[k].im);  // proj_lie(-UA) = -proj_lie(UA)
     }
-    M3<R> X;
+    AntiH<R> X;
     if (STAGE == 1) {
-        const R c1 = (R)(0.25 * eps);
-#pragma unroll
-        for (int k = 0; k < 9; k++) X.e[k] = scl(c1, F.e[k]);
+        X = scl((R)(0.25 * eps), F);
         Z.store(mu, par, h, F);
     } else if (STAGE == 2) {
-        M3<R> z0 = Z.load(mu, par, h);
-        const R a = (R)((8.0 / 9.0) * eps), b = (R)((17.0 / 36.0) * eps);
-        const R a1 = (R)(8.0 / 9.0), b1 = (R)(17.0 / 36.0);
-        M3<R> zn;
-#pragma unroll
-        for (int k = 0; k < 9; k++) {
-            X.e[k] = scl(a, F.e[k]) - scl(b, z0.e[k]);
-            zn.e[k] = scl(a1, F.e[k]) - scl(b1, z0.e[k]);
-        }
+        const AntiH<R> z0 = Z.load(mu, par, h);
+        // X = eps (8/9 F - 17/36 Z) and the new Z = 8/9 F - 17/36 Z
+        const AntiH<R> zn = axpby((R)(8.0 / 9.0), F, (R)(-17.0 / 36.0), z0);
+        X = scl((R)eps, zn);
         Z.store(mu, par, h, zn);
     } else {
-        M3<R> z0 = Z.load(mu, par, h);
-        const R a = (R)(0.75 * eps), b = (R)eps;
-#pragma unroll
-        for (int k = 0; k < 9; k++) X.e[k] = scl(a, F.e[k]) - scl(b, z0.e[k]);
+        X = axpby((R)(0.75 * eps), F, (R)(-eps), Z.load(mu, par, h));
     }
     M3<R> E = exp_su3(X);
     M3<R> w = mul_nn(E, u);
@@ -944,45 +906,66 @@ __device__ __forceinline__ void flow_link(const Geom& g, const LinkField<R, NE>&
     Wout.store(mu, par, h, w);
 }
 
-// Single-lattice RK3 stage.  Grid: blockIdx.x = (site block) * 8 + (mu*2 + parity), so the 8
-// link classes of a block of sites run together and share their neighbour links in L2.
+// Links of a block of the flow kernels.  FP64: the four warps take the four directions of one tile of
+// 32 half-sites of one parity (blockIdx.x = 2 * tile + parity), so that they read the same neighbour
+// links and share them in L1: with one (mu, parity) class of 128 half-sites a block, each link came
+// from L2 for every use (19 links a link, 10 GB a 32^4 stage at 60% of the L2 rate); L1 now serves 31%
+// of the sectors and a stage takes 649-660 against 695 us (24^4: 185 against 190).  FP32 kernels, bound
+// by issue, keep one class a block (blockIdx.x = 8 * site block + mu * 2 + parity): the direction is
+// then uniform over the block (16^4: 30.6 against 31.6 us).
+template <typename R>
+__device__ __forceinline__ void flow_map(unsigned b, int& mu, int& par, int64_t& h) {
+    if constexpr (sizeof(R) == 8) {
+        mu = threadIdx.x >> 5;
+        par = b & 1;
+        h = (int64_t)(b >> 1) * 32 + (threadIdx.x & 31);
+    } else {
+        mu = (b & 7) >> 1;
+        par = b & 1;
+        h = (int64_t)(b >> 3) * QCB_FLOW_THREADS + threadIdx.x;
+    }
+}
+
+// Single-lattice RK3 stage.  The 8 link classes of a range of sites run together (flow_map) and share
+// their neighbour links in L2.
 template <typename R, int NE, int STAGE>
-__global__ void __launch_bounds__(QCB_FLOW1_THREADS, QCB_FLOW1_MINB(R))
+__global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW1_MINB(R))
     k_flow_stage(Geom g, LinkField<R, NE> Win, LinkField<R, NE> Wout, AlgField<R> Z, double eps, int reproject) {
-    const int lt = blockIdx.x & 7;
-    const int64_t h = (int64_t)(blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+    int mu, par;
+    int64_t h;
+    flow_map<R>(blockIdx.x, mu, par, h);
     if (h >= g.Vh) return;
-    flow_link<R, NE, STAGE>(g, Win, Wout, Z, eps, lt >> 1, lt & 1, (int)h, reproject);
+    flow_link<R, NE, STAGE>(g, Win, Wout, Z, eps, mu, par, (int)h, reproject);
 }
 
 // Stage 1 that also writes the clover halves of its input configuration (the measurement of a
 // measured flow step; k_clover_halves completes it).  The links it writes are those of
 // k_flow_stage<R, NE, 1>, bit for bit.
 template <typename R, int NE>
-__global__ void __launch_bounds__(QCB_FLOW1_THREADS, QCB_FLOW_MEAS_MINB(R))
+__global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MEAS_MINB(R))
     k_flow_stage1_meas(Geom g, LinkField<R, NE> Win, LinkField<R, NE> Wout, AlgField<R> Z, double eps, int reproject,
                        HalfClovers<R> H) {
-    const int lt = blockIdx.x & 7;
-    const int64_t h = (int64_t)(blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+    int mu, par;
+    int64_t h;
+    flow_map<R>(blockIdx.x, mu, par, h);
     if (h >= g.Vh) return;
-    flow_link<R, NE, 1, true>(g, Win, Wout, Z, eps, lt >> 1, lt & 1, (int)h, reproject, H);
+    flow_link<R, NE, 1, true>(g, Win, Wout, Z, eps, mu, par, (int)h, reproject, H);
 }
 
 // ------------------------------------------------------------------ the reference's separate flow passes
 // GradientFlow's member passes (src/flow/gradient_flow.cpp:17-121), for callers that drive them one
 // by one; rk3_step runs the fused stages above.  Forces are su(3) fields in the accumulator layout.
-// compute_force: F = proj_lie_su3(-U A) of every link, with the fused stage's staple and projection.
-// Grid: blockIdx.x = (site block) * 8 + (mu*2 + parity), as the fused stage.
+// compute_force: F = proj_lie_su3(-U A) of every link, with the fused stage's staple, projection and grid.
 template <typename R, int NE>
-__global__ void __launch_bounds__(QCB_FLOW1_THREADS) k_flow_force(Geom g, LinkField<R, NE> W, AlgField<R> F) {
-    const int lt = blockIdx.x & 7;
-    const int64_t h = (int64_t)(blockIdx.x >> 3) * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(QCB_FLOW_THREADS) k_flow_force(Geom g, LinkField<R, NE> W, AlgField<R> F) {
+    int mu, par;
+    int64_t h;
+    flow_map<R>(blockIdx.x, mu, par, h);
     if (h >= g.Vh) return;
-    const int mu = lt >> 1, par = lt & 1;
     int c[4];
     site_coords(g, par, (uint32_t)h, c);
     const int lex = lex_of(g, c);
-    const M3<R> A = staple_rt_rows<R, NE>(g, W, c, lex, par, mu);
+    const M3<R> A = staple_rt_rows<R, NE, true>(g, W, c, lex, par, mu);
     const M3<R> u = W.load_ro(mu, par, (int)h);
     F.store(mu, par, (int)h, neg_proj_lie_mul(u, A));
 }
@@ -996,16 +979,8 @@ __global__ void __launch_bounds__(256) k_flow_update(Geom g, LinkField<R, NE> W,
     const int lt = blockIdx.y, mu = lt >> 1, par = lt & 1;
     const int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= g.Vh) return;
-    const M3<R> z0 = F0.load(mu, par, (int)h);
-    M3<R> X;
-    if (use_f1) {
-        const M3<R> z1 = F1.load(mu, par, (int)h);
-#pragma unroll
-        for (int k = 0; k < 9; k++) X.e[k] = scl((R)a, z1.e[k]) - scl((R)b, z0.e[k]);
-    } else {
-#pragma unroll
-        for (int k = 0; k < 9; k++) X.e[k] = scl((R)a, z0.e[k]);
-    }
+    const AntiH<R> z0 = F0.load(mu, par, (int)h);
+    const AntiH<R> X = use_f1 ? axpby((R)a, F1.load(mu, par, (int)h), (R)-b, z0) : scl((R)a, z0);
     M3<R> w = mul_nn(exp_su3(X), W.load(mu, par, (int)h));
     if (reproject) reproject_fp64(w);
     W.store(mu, par, (int)h, w);
@@ -1017,11 +992,7 @@ __global__ void __launch_bounds__(256) k_flow_replace(int64_t Vh, AlgField<R> F0
     const int lt = blockIdx.y, mu = lt >> 1, par = lt & 1;
     const int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= Vh) return;
-    const M3<R> z0 = F0.load(mu, par, (int)h), z1 = F1.load(mu, par, (int)h);
-    const R a1 = (R)(8.0 / 9.0), b1 = (R)(17.0 / 36.0);
-    M3<R> zn;
-#pragma unroll
-    for (int k = 0; k < 9; k++) zn.e[k] = scl(a1, z1.e[k]) - scl(b1, z0.e[k]);
+    const AntiH<R> zn = axpby((R)(8.0 / 9.0), F1.load(mu, par, (int)h), (R)(-17.0 / 36.0), F0.load(mu, par, (int)h));
     F0.store(mu, par, (int)h, zn);
 }
 

@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
 }
 
 // ---------------------------------------------------------------- flow, one RK3 stage
-// Tile classes interleave the 8 (mu, parity) link classes of a block of sites so that they
+// The 8 tiles of a block of sites interleave its (mu, parity) link classes (flow_map) so that they
 // share their neighbour links in L2.  With f = flip ^ flip_xor, the input of stage s is links
 // when (f + s - 1) is even; a whole RK3 step therefore moves the field to the other buffer.
 template <typename R, int NE, int STAGE>
@@ -79,9 +79,9 @@ __global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MINB(R))
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const LatDesc* d = lattice_of(lats, tile_lat, one, t >> 3);
         const Geom g = d->g;
-        const int lt = t - 8 * d->nb_begin;
-        const int cls = lt & 7;
-        const int h = (lt >> 3) * TILE + threadIdx.x;
+        int mu, par;
+        int64_t h;
+        flow_map<R>(t - 8 * d->nb_begin, mu, par, h);
         if (h >= g.Vh) continue;
         const bool in_b = (((d->flip ^ flip_xor) + STAGE - 1) & 1) != 0;
         const LinkField<R, NE> win = lview<R, NE>(in_b ? d->links_out : d->links, g.Vh);
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MINB(R))
         AlgField<R> z;
         z.p = (typename AlgField<R>::C2*)d->z;
         z.Vh = g.Vh;
-        flow_link<R, NE, STAGE>(g, win, wout, z, d->eps, cls >> 1, cls & 1, h, reproject);
+        flow_link<R, NE, STAGE>(g, win, wout, z, d->eps, mu, par, (int)h, reproject);
     }
 }
 
@@ -102,9 +102,9 @@ __global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MEAS_MINB(R))
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const LatDesc* d = lattice_of(lats, tile_lat, one, t >> 3);
         const Geom g = d->g;
-        const int lt = t - 8 * d->nb_begin;
-        const int cls = lt & 7;
-        const int h = (lt >> 3) * TILE + threadIdx.x;
+        int mu, par;
+        int64_t h;
+        flow_map<R>(t - 8 * d->nb_begin, mu, par, h);
         if (h >= g.Vh) continue;
         const bool in_b = ((d->flip ^ flip_xor) & 1) != 0;
         const LinkField<R, NE> win = lview<R, NE>(in_b ? d->links_out : d->links, g.Vh);
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MEAS_MINB(R))
         z.p = (typename AlgField<R>::C2*)d->z;
         z.Vh = g.Vh;
         const HalfClovers<R> H{(R*)d->halves, 2 * g.Vh};
-        flow_link<R, NE, 1, true>(g, win, wout, z, d->eps, cls >> 1, cls & 1, h, reproject, H);
+        flow_link<R, NE, 1, true>(g, win, wout, z, d->eps, mu, par, (int)h, reproject, H);
     }
 }
 
