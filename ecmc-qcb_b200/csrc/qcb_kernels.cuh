@@ -135,8 +135,8 @@ __device__ __forceinline__ M3<R> staple_rt(const Geom& g, const LinkField<R, NE>
 // rows 0-1 of t^dag need columns 0-1 of t only.  That is 42 instead of 54 complex
 // multiply-adds a staple.  The rebuilt row differs from the explicit product by the
 // links' distance from SU(3), which in FP32 storage is the FP32 rounding level (~1e-7).
-// FLOW: the flow kernels' order of nu, mu ^ 1, mu ^ 2, mu ^ 3, in which the warps of mu and nu are in the
-// same plane at the same time and share its links in L1; else ascending, as compute_staple.
+// FLOW: the FP64 flow kernels' order of nu, mu ^ 1, mu ^ 2, mu ^ 3, in which the warps of mu and nu are in
+// the same plane at the same time and share its links in L1; else ascending, as compute_staple.
 template <typename R, int NE, bool FLOW = false>
 __device__ __forceinline__ M3<R> staple_rt_rows(const Geom& g, const LinkField<R, NE>& U, const int c[4],
                                                 int lex, int par, int mu) {
@@ -304,7 +304,7 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
     const int64_t site = (int64_t)par * g.Vh + (lex >> 1), site_up = (int64_t)opp * g.Vh + (xmu >> 1);
 #pragma unroll 1
     for (int k = 0; k < 3; k++) {
-        const int nu = mu ^ (k + 1);
+        const int nu = sizeof(R) == 8 ? mu ^ (k + 1) : (k < mu ? k : k + 1);
         const int plane = mu < nu ? plane_index(mu, nu) : plane_index(nu, mu);
         const bool owned = plane_owner(plane) == mu;
         const int dnu = sel4(st.dn, nu);
@@ -421,7 +421,7 @@ __device__ __forceinline__ AntiH<R> neg_proj_lie_mul(const M3<R>& u, const M3<R>
         }
         F.o[k] = mkc<R>(R(0.5) * (w.re - v.re), R(-0.5) * (v.im + w.im));
     }
-    const R tr3 = (im[0] + im[1] + im[2]) * R(1.0 / 3.0);
+    const R tr3 = (im[0] + im[1] + im[2]) / R(3);
 #pragma unroll
     for (int i = 0; i < 3; i++) F.d[i] = tr3 - im[i];
     return F;
@@ -881,7 +881,7 @@ __device__ __forceinline__ void flow_link(const Geom& g, const LinkField<R, NE>&
         }
     } else {
         // two-row staple products and the projection's entries only
-        const M3<R> A = staple_rt_rows<R, NE, true>(g, Win, c, lex, par, mu);
+        const M3<R> A = staple_rt_rows<R, NE, sizeof(R) == 8>(g, Win, c, lex, par, mu);
         u = Win.load_ro(mu, par, h);
         F = neg_proj_lie_mul(u, A);
     }
@@ -891,10 +891,8 @@ __device__ __forceinline__ void flow_link(const Geom& g, const LinkField<R, NE>&
         Z.store(mu, par, h, F);
     } else if (STAGE == 2) {
         const AntiH<R> z0 = Z.load(mu, par, h);
-        // X = eps (8/9 F - 17/36 Z) and the new Z = 8/9 F - 17/36 Z
-        const AntiH<R> zn = axpby((R)(8.0 / 9.0), F, (R)(-17.0 / 36.0), z0);
-        X = scl((R)eps, zn);
-        Z.store(mu, par, h, zn);
+        X = axpby((R)((8.0 / 9.0) * eps), F, (R)(-(17.0 / 36.0) * eps), z0);
+        Z.store(mu, par, h, axpby((R)(8.0 / 9.0), F, (R)(-17.0 / 36.0), z0));
     } else {
         X = axpby((R)(0.75 * eps), F, (R)(-eps), Z.load(mu, par, h));
     }
@@ -965,7 +963,7 @@ __global__ void __launch_bounds__(QCB_FLOW_THREADS) k_flow_force(Geom g, LinkFie
     int c[4];
     site_coords(g, par, (uint32_t)h, c);
     const int lex = lex_of(g, c);
-    const M3<R> A = staple_rt_rows<R, NE, true>(g, W, c, lex, par, mu);
+    const M3<R> A = staple_rt_rows<R, NE, sizeof(R) == 8>(g, W, c, lex, par, mu);
     const M3<R> u = W.load_ro(mu, par, (int)h);
     F.store(mu, par, (int)h, neg_proj_lie_mul(u, A));
 }

@@ -287,11 +287,10 @@ QCB_HD void ch_coeffs(double t, double d, double q[6]) {
 //   t = |X01|^2 + |X02|^2 + |X12|^2 + (a0^2 + a1^2 + a2^2)/2,
 //   d = det H = a0 a1 a2 + 2 Im(X01 X12 conj(X02)) - a0 |X12|^2 - a1 |X02|^2 - a2 |X01|^2  (X = iH)
 // and the recurrence run in double for every storage precision R (the "Cayley-Hamilton coefficients
-// in FP64" rule); the matrix part runs in R.  X^2 is Hermitian: its diagonal is -(a_i^2 + the |o|^2
-// of row i) and X2_01 = i (a0 + a1) X01 - X02 conj(X12) and so on.  Working on the nine
-// reals takes about 100 multiply-adds less than full 3x3 products, the flow stages' bound in FP64
-// (pipe) and FP32 (issue): together with the shorter recurrence a 32^4 stage takes 637 against
-// 649 us FP64-18, 615 against 641 us FP64-12 and 360 against 374 us FP32-12.
+// in FP64" rule); the matrix part runs in R.  X^2 and the sum are formed from the nine reals with the
+// terms and their order of full 3x3 products, less those that an exactly zero real diagonal makes
+// zero: the same result in about 60 multiply-adds less, for the flow stages' bound in FP64 (pipe) and
+// FP32 (issue).
 template <typename R>
 QCB_HD M3<R> exp_su3(const AntiH<R>& X) {
     const Cx<R>* o = X.o;
@@ -311,30 +310,37 @@ QCB_HD M3<R> exp_su3(const AntiH<R>& X) {
     double q[6];
     ch_coeffs(t, d, q);
     const Cx<R> q0 = mkc<R>((R)q[0], (R)q[1]), q1 = mkc<R>((R)q[2], (R)q[3]), q2 = mkc<R>((R)q[4], (R)q[5]);
-    const R n01 = fma(o[0].re, o[0].re, o[0].im * o[0].im), n02 = fma(o[1].re, o[1].re, o[1].im * o[1].im);
-    const R n12 = fma(o[2].re, o[2].re, o[2].im * o[2].im);
-    const R s[3] = {-fma(a[0], a[0], n01 + n02), -fma(a[1], a[1], n01 + n12), -fma(a[2], a[2], n02 + n12)};
-    // X2_01, X2_02, X2_12
-    const R a01 = a[0] + a[1], a02 = a[0] + a[2], a12 = a[1] + a[2];
-    Cx<R> x2[3] = {mkc<R>(-a01 * o[0].im, a01 * o[0].re), mkc<R>(-a02 * o[1].im, a02 * o[1].re),
-                   mkc<R>(-a12 * o[2].im, a12 * o[2].re)};
+    // -|z|^2 added to r
+    auto sub_norm = [](Cx<R> z, R r) { return fma(-z.re, z.re, fma(-z.im, z.im, r)); };
+    const R s[3] = {sub_norm(o[1], sub_norm(o[0], -(a[0] * a[0]))),
+                    sub_norm(o[2], fma(-a[1], a[1], fma(-o[0].re, o[0].re, -(o[0].im * o[0].im)))),
+                    fma(-a[2], a[2], sub_norm(o[2], fma(-o[1].re, o[1].re, -(o[1].im * o[1].im))))};
+    Cx<R> x2[3];  // (X^2)_01, (X^2)_02, (X^2)_12
+    x2[0].re = fma(-o[0].im, a[1], -(a[0] * o[0].im));
+    x2[0].im = fma(o[0].re, a[1], a[0] * o[0].re);
     x2[0].re = fma(-o[1].re, o[2].re, fma(-o[1].im, o[2].im, x2[0].re));
-    x2[0].im = fma(-o[1].im, o[2].re, fma(o[1].re, o[2].im, x2[0].im));
+    x2[0].im = fma(o[1].re, o[2].im, fma(-o[1].im, o[2].re, x2[0].im));
+    x2[1] = mkc<R>(-(a[0] * o[1].im), a[0] * o[1].re);
     cmac(x2[1], o[0], o[2]);
-    x2[2].re = fma(-o[0].re, o[1].re, fma(-o[0].im, o[1].im, x2[2].re));
-    x2[2].im = fma(-o[0].re, o[1].im, fma(o[0].im, o[1].re, x2[2].im));
+    x2[1].re = fma(-o[1].im, a[2], x2[1].re);
+    x2[1].im = fma(o[1].re, a[2], x2[1].im);
+    x2[2].re = fma(-o[0].re, o[1].re, -(o[0].im * o[1].im));
+    x2[2].im = fma(-o[0].re, o[1].im, o[0].im * o[1].re);
+    x2[2].re = fma(-o[2].im, a[2], fma(-a[1], o[2].im, x2[2].re));
+    x2[2].im = fma(o[2].re, a[2], fma(a[1], o[2].re, x2[2].im));
     M3<R> E;
 #pragma unroll
     for (int i = 0; i < 3; i++)
-        E(i, i) = mkc<R>(fma(q2.re, s[i], fma(-q1.im, a[i], q0.re)), fma(q2.im, s[i], fma(q1.re, a[i], q0.im)));
+        E(i, i) = mkc<R>(fma(q2.re, s[i], -(q1.im * a[i])) + q0.re, fma(q2.im, s[i], q1.re * a[i]) + q0.im);
     const int I[3] = {0, 0, 1}, J[3] = {1, 2, 2};
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         // E_ij = q1 X_ij + q2 X2_ij, E_ji = -q1 conj(X_ij) + q2 conj(X2_ij)
-        Cx<R> u = q1 * o[k];
+        Cx<R> u = mkc<R>(fma(q1.re, o[k].re, -(q1.im * o[k].im)), fma(q1.im, o[k].re, q1.re * o[k].im));
         cmac(u, q2, x2[k]);
-        Cx<R> w = mkc<R>(fma(-q1.re, o[k].re, -q1.im * o[k].im), fma(q1.re, o[k].im, -q1.im * o[k].re));
-        cmac_nc(w, q2, x2[k]);
+        Cx<R> w = mkc<R>(fma(-q1.re, o[k].re, -(q1.im * o[k].im)), fma(-q1.im, o[k].re, q1.re * o[k].im));
+        w.re = fma(q2.re, x2[k].re, fma(q2.im, x2[k].im, w.re));
+        w.im = fma(-q2.re, x2[k].im, fma(q2.im, x2[k].re, w.im));
         E(I[k], J[k]) = u;
         E(J[k], I[k]) = w;
     }
