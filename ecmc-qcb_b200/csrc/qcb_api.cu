@@ -147,8 +147,6 @@ int check_err_flag(qcb_field_s* f) {
     CK(cudaStreamSynchronize(f->stream));
     if (h) {
         CK(cudaMemsetAsync(f->d_err, 0, sizeof(int), f->stream));
-        if (h & DERR_BULK_WAIT)
-            return fail(QCB_ETIMEOUT, "heatbath: bulk copy of the block's links did not complete (links left unchanged)");
         if (h & DERR_KP_SCALE)
             return fail(QCB_ERANGE, "heatbath: zero or non-finite SU(2) projection of the staple (link left unchanged)");
         return fail(QCB_ERANGE, "heatbath: Kennedy-Pendleton attempt cap (2^20) reached (link left unchanged)");

@@ -28,6 +28,23 @@ struct FmtImpl {
         return *cache;
     }
 
+    // Launch of a kernel that begins with work of its own and then waits for the launches before it
+    // (cudaGridDependencySynchronize): its blocks may start when those of the previous launch have
+    // ended or have said that they may, without the gap between two launches in a stream.
+    template <typename... P, typename... A>
+    static cudaError_t launch_early(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, A... a) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(block);
+        cfg.stream = s;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
+    }
+
     template <int MU, int BLOCK, int MINB>
     static cudaError_t hb_launch(const WorkList& w, int par, int n_hits, const uint32_t* sweep_dev, uint32_t sweep_add,
                                  int reproject, int* err, cudaStream_t s) {
@@ -76,10 +93,14 @@ struct FmtImpl {
     template <int MU>
     static cudaError_t hb1_mu(const Geom& g, void* links, int par, double c_alpha, int n_hits, uint64_t seed,
                               uint32_t sweep, int rep, int* err, cudaStream_t s) {
+        if constexpr (sizeof(R) == 8)
+            if (g.Vh <= kHbGroupMaxVh)
+                return launch_early(k_hb_group<NE, MU>, (unsigned)((g.Vh + kHbGroupLinks - 1) / kHbGroupLinks),
+                                    kHbLanes * kHbGroupLinks, s, g, view(links, g.Vh), par, c_alpha, n_hits, seed,
+                                    sweep, rep, err);
         const unsigned nb = (unsigned)((g.Vh + QCB_HB_THREADS - 1) / QCB_HB_THREADS);
-        k_hb_subsweep<R, NE, MU><<<nb, QCB_HB_THREADS, 0, s>>>(g, view(links, g.Vh), par, c_alpha, n_hits, seed, sweep,
-                                                               rep, err);
-        return cudaGetLastError();
+        return launch_early(k_hb_subsweep<R, NE, MU>, nb, QCB_HB_THREADS, s, g, view(links, g.Vh), par, c_alpha, n_hits,
+                            seed, sweep, rep, err);
     }
     static cudaError_t hb1(const Geom& g, void* links, int par, int mu, double c_alpha, int n_hits, uint64_t seed,
                            uint32_t sweep, int rep, int* err, cudaStream_t s) {

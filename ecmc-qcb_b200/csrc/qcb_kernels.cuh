@@ -12,41 +12,7 @@ namespace qcb {
 constexpr double kPi = 3.14159265358979323846;
 
 // Device error flags (bit mask written by kernels, read by the host after a sync).
-enum : int { DERR_KP_CAP = 1, DERR_KP_SCALE = 2, DERR_BULK_WAIT = 4 };
-
-// ------------------------------------------------------------------ bulk copies into shared memory
-// One-shot mbarrier-tracked bulk copies (the TMA engine's cp.async.bulk, global -> this CTA's shared
-// memory, no multicast).  Addresses 16-byte aligned, sizes multiples of 16 bytes.
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst), b = (unsigned)__cvta_generic_to_shared(bar);
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d),
-                 "l"(src), "r"(bytes), "r"(b)
-                 : "memory");
-}
-// Waits for phase `phase` of the barrier, at most max_tries polls (each poll may suspend the thread
-// for a bounded, hardware-chosen time); false if the copies did not land in that time.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned phase, int max_tries) {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
-    for (int i = 0; i < max_tries; i++) {
-        unsigned ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(ok)
-            : "r"(a), "r"(phase)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
+enum : int { DERR_KP_CAP = 1, DERR_KP_SCALE = 2 };
 
 // byte reversal of a double (ILDG files are big-endian, src/io/ildg.cpp:25-32)
 __device__ __forceinline__ double bswap_f64(double x) {
@@ -437,9 +403,6 @@ __device__ __forceinline__ AntiH<R> neg_proj_lie_mul(const M3<R>& u, const M3<R>
 #ifndef QCB_HB_MINB
 #define QCB_HB_MINB(R) (sizeof(R) == 8 ? 4 : 6)
 #endif
-#ifndef QCB_HB_BULK_LINKS
-#define QCB_HB_BULK_LINKS 0
-#endif
 #ifndef QCB_FLOW_THREADS
 #define QCB_FLOW_THREADS 128
 #endif
@@ -491,6 +454,32 @@ __device__ __forceinline__ KPDraws kp_draws_at(const LinkStream& rng, uint32_t n
     return d;
 }
 
+// The direction draws (u_phi, u_cos) of a subgroup element as the angles' sines and cosines.
+struct KPDir {
+    double st, ct, sp, cp;
+};
+__device__ __forceinline__ KPDir kp_direction(double2 F) {
+    KPDir d;
+    d.ct = 2.0 * F.y - 1.0;
+    d.st = sqrt(1.0 - d.ct * d.ct);
+    sincospi(2.0 * F.x, &d.sp, &d.cp);
+    return d;
+}
+// mult(x, adj(v))  (src/su3/utils.cpp:53-63) for the accepted x = (a0, sqrt(1 - a0^2) n)
+__device__ __forceinline__ Quat kp_element(double a0, const KPDir& d, const Quat& v) {
+    const double rs = sqrt(1.0 - a0 * a0);
+    const Quat x = {a0, rs * d.st * d.cp, rs * d.st * d.sp, rs * d.ct};
+    return Quat{x.a0 * v.a0 + x.a1 * v.a1 + x.a2 * v.a2 + x.a3 * v.a3,
+                -x.a0 * v.a1 + x.a1 * v.a0 - x.a2 * v.a3 + x.a3 * v.a2,
+                -x.a0 * v.a2 + x.a1 * v.a3 + x.a2 * v.a0 - x.a3 * v.a1,
+                -x.a0 * v.a3 - x.a1 * v.a2 + x.a2 * v.a1 + x.a3 * v.a0};
+}
+// log r1 + cos^2(2 pi r2) log r3 of an attempt's draws; the attempt's lambda^2 is -0.5/alpha times it
+__device__ __forceinline__ double kp_log(double r1, double r2, double r3) {
+    const double c = cospi(2.0 * r2);
+    return __dadd_rn(log(r1), __dmul_rn(__dmul_rn(c, c), log(r3)));
+}
+
 // generate_su2_kp (src/heatbath/heatbath.cpp:8-36) + su2_step (:39-44), drawing in the
 // reference's order: (delta, r1, r2, r3) per Kennedy-Pendleton attempt, then (u_phi, u_cos).
 // With c_alpha = -0.75/beta, -0.5/alpha = c_alpha / k (alpha = 2 beta k / 3), so one rsqrt
@@ -516,10 +505,8 @@ __device__ __forceinline__ Quat su2_step(double c_alpha, Quat w, const LinkStrea
     double2 P = d.P, Q = d.Q, F = d.F;
     int it = 0;
     for (; it < cap; it++) {
-        const double delta = P.x, r1 = P.y, r2 = Q.x, r3 = Q.y;
-        double c = cospi(2.0 * r2);
-        double lsq = __dmul_rn(m05a, __dadd_rn(log(r1), __dmul_rn(__dmul_rn(c, c), log(r3))));
-        if (__dmul_rn(delta, delta) <= __dadd_rn(1.0, -lsq)) {
+        const double lsq = __dmul_rn(m05a, kp_log(P.y, Q.x, Q.y));
+        if (__dmul_rn(P.x, P.x) <= __dadd_rn(1.0, -lsq)) {
             a0 = __dadd_rn(1.0, -__dmul_rn(2.0, lsq));
             ok = true;
             break;
@@ -536,25 +523,12 @@ __device__ __forceinline__ Quat su2_step(double c_alpha, Quat w, const LinkStrea
         atomicOr(err, cap > 0 ? (int)DERR_KP_CAP : (int)DERR_KP_SCALE);
         return Quat{1.0, 0.0, 0.0, 0.0};
     }
-    const double rs = sqrt(1.0 - a0 * a0);
-    const double uphi = F.x;
-    const double cos_t = 2.0 * F.y - 1.0;
-    const double sin_t = sqrt(1.0 - cos_t * cos_t);
-    double sp, cp;
-    sincospi(2.0 * uphi, &sp, &cp);
-    const Quat x = {a0, rs * sin_t * cp, rs * sin_t * sp, rs * cos_t};
-    // mult(x, adj(v))  (src/su3/utils.cpp:53-63)
-    return Quat{x.a0 * v.a0 + x.a1 * v.a1 + x.a2 * v.a2 + x.a3 * v.a3,
-                -x.a0 * v.a1 + x.a1 * v.a0 - x.a2 * v.a3 + x.a3 * v.a2,
-                -x.a0 * v.a2 + x.a1 * v.a3 + x.a2 * v.a0 - x.a3 * v.a1,
-                -x.a0 * v.a3 - x.a1 * v.a2 + x.a2 * v.a1 + x.a3 * v.a0};
+    return kp_element(a0, kp_direction(F), v);
 }
 
-// One Cabibbo-Marinari subgroup update of u in place (src/heatbath/heatbath_mpi.cpp:14-32):
-// w = quaternion of the (I,J) block of W = u*A, r = su2_step(w), u <- embed_{IJ}(r) * u.
+// Quaternion of the (I,J) block of W = u A (su2_to_quaternion, src/su3/utils.cpp:47-50).
 template <typename R, int I, int J, typename AM>
-__device__ __forceinline__ void cm_subgroup(M3<R>& u, const AM& A, double c_alpha, const LinkStream& rng, KPDraws& d,
-                                            bool more, int* err) {
+__device__ __forceinline__ Quat cm_quaternion(const M3<R>& u, const AM& A) {
     Cx<R> wii = mkc<R>(0, 0), wij = mkc<R>(0, 0), wji = mkc<R>(0, 0), wjj = mkc<R>(0, 0);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -563,16 +537,17 @@ __device__ __forceinline__ void cm_subgroup(M3<R>& u, const AM& A, double c_alph
         cmac(wji, u(J, k), A(k, I));
         cmac(wjj, u(J, k), A(k, J));
     }
-    // su2_to_quaternion (src/su3/utils.cpp:47-50)
-    Quat w = {((double)wii.re + (double)wjj.re) / 2.0, ((double)wij.im + (double)wji.im) / 2.0,
-              ((double)wij.re - (double)wji.re) / 2.0, ((double)wii.im - (double)wjj.im) / 2.0};
-    Quat r = su2_step(c_alpha, w, rng, d, more, err);
-    // su2_quaternion_to_su3 (src/su3/utils.cpp:33-44) applied from the left
-    Cx<R> rii = mkc<R>((R)r.a0, (R)r.a3), rjj = mkc<R>((R)r.a0, (R)-r.a3);
-    Cx<R> rij = mkc<R>((R)r.a2, (R)r.a1), rji = mkc<R>((R)-r.a2, (R)r.a1);
+    return Quat{((double)wii.re + (double)wjj.re) / 2.0, ((double)wij.im + (double)wji.im) / 2.0,
+                ((double)wij.re - (double)wji.re) / 2.0, ((double)wii.im - (double)wjj.im) / 2.0};
+}
+// u <- embed_{IJ}(r) u (su2_quaternion_to_su3, src/su3/utils.cpp:33-44, applied from the left).
+template <typename R, int I, int J>
+__device__ __forceinline__ void cm_apply(M3<R>& u, const Quat& r) {
+    const Cx<R> rii = mkc<R>((R)r.a0, (R)r.a3), rjj = mkc<R>((R)r.a0, (R)-r.a3);
+    const Cx<R> rij = mkc<R>((R)r.a2, (R)r.a1), rji = mkc<R>((R)-r.a2, (R)r.a1);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        Cx<R> ui = u(I, k), uj = u(J, k);
+        const Cx<R> ui = u(I, k), uj = u(J, k);
         Cx<R> ni = rii * ui;
         cmac(ni, rij, uj);
         Cx<R> nj = rji * ui;
@@ -580,6 +555,15 @@ __device__ __forceinline__ void cm_subgroup(M3<R>& u, const AM& A, double c_alph
         u(I, k) = ni;
         u(J, k) = nj;
     }
+}
+
+// One Cabibbo-Marinari subgroup update of u in place (src/heatbath/heatbath_mpi.cpp:14-32):
+// w = quaternion of the (I,J) block of W = u*A, r = su2_step(w), u <- embed_{IJ}(r) * u.
+template <typename R, int I, int J, typename AM>
+__device__ __forceinline__ void cm_subgroup(M3<R>& u, const AM& A, double c_alpha, const LinkStream& rng, KPDraws& d,
+                                            bool more, int* err) {
+    const Quat w = cm_quaternion<R, I, J>(u, A);
+    cm_apply<R, I, J>(u, su2_step(c_alpha, w, rng, d, more, err));
 }
 
 // A thread's staple held in shared memory for the hits: element k of the thread's matrix at
@@ -621,8 +605,8 @@ struct StapleSlot {
 
 // staple_rt_rows accumulated into a shared-memory slot instead of registers: each forward or
 // backward staple is formed in registers and added to the slot, so the 18-real accumulator does not
-// occupy registers across the nu loop.
-template <typename R, int NE>
+// occupy registers across the nu loop.  RO: read-only loads (no launch that runs meanwhile writes U).
+template <typename R, int NE, bool RO = true>
 __device__ __forceinline__ void staple_rows_into(const Geom& g, const LinkField<R, NE>& U, const int c[4], int lex,
                                                  int par, int mu, const StapleSlot<R>& S) {
 #pragma unroll
@@ -648,8 +632,8 @@ __device__ __forceinline__ void staple_rows_into(const Geom& g, const LinkField<
         const int xmnu = lex + dnu;
         const int xmumnu = xmu + dnu;
         {
-            const M3<R> a = U.load_ro(nu, opp, xmu >> 1);
-            const M3<R> b = U.load_ro(mu, opp, xnu >> 1);
+            const M3<R> a = U.template load_t<RO>(nu, opp, xmu >> 1);
+            const M3<R> b = U.template load_t<RO>(mu, opp, xnu >> 1);
             Cx<R> t[2][3], r[2][3];
 #pragma unroll
             for (int i = 0; i < 2; i++)
@@ -659,7 +643,7 @@ __device__ __forceinline__ void staple_rows_into(const Geom& g, const LinkField<
 #pragma unroll
                     for (int q = 0; q < 3; q++) cmac_nc(t[i][j], a(i, q), b(j, q));
                 }
-            const M3<R> d = U.load_ro(nu, par, lex >> 1);
+            const M3<R> d = U.template load_t<RO>(nu, par, lex >> 1);
 #pragma unroll
             for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -671,8 +655,8 @@ __device__ __forceinline__ void staple_rows_into(const Geom& g, const LinkField<
             add_rows(r);
         }
         {
-            const M3<R> v1 = U.load_ro(mu, opp, xmnu >> 1);
-            const M3<R> v0 = U.load_ro(nu, par, xmumnu >> 1);
+            const M3<R> v1 = U.template load_t<RO>(mu, opp, xmnu >> 1);
+            const M3<R> v0 = U.template load_t<RO>(nu, par, xmumnu >> 1);
             Cx<R> t[3][2], r[2][3];
 #pragma unroll
             for (int i = 0; i < 3; i++)
@@ -682,7 +666,7 @@ __device__ __forceinline__ void staple_rows_into(const Geom& g, const LinkField<
 #pragma unroll
                     for (int q = 0; q < 3; q++) cmac(t[i][j], v1(i, q), v0(q, j));
                 }
-            const M3<R> v2 = U.load_ro(nu, opp, xmnu >> 1);
+            const M3<R> v2 = U.template load_t<RO>(nu, opp, xmnu >> 1);
 #pragma unroll
             for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -748,10 +732,12 @@ __device__ __forceinline__ void cm_subgroup_rt(const StapleSlot<R>& u, const Sta
 // 32^4 FP64 sub-sweep at N_hits = 2 against 0.235 ms with the staple in registers).  Without a
 // slot (blocks too large for the static shared memory) the three subgroups are unrolled on
 // register-resident matrices.
-template <typename R, int NE, int MU, bool SLOT>
+// EARLY (k_hb_subsweep's launches): the first draws, then the wait for the previous launch; the links are
+// then loaded as ordinary memory, since the previous launch may still be writing when this one starts.
+template <typename R, int NE, int MU, bool SLOT, bool EARLY = false>
 __device__ __forceinline__ void hb_link(const Geom& g, const LinkField<R, NE>& U, int par, int h, double c_alpha,
                                         int n_hits, uint64_t seed, uint32_t sweep, int reproject, int* err,
-                                        typename V2<R>::T* slot, int slot_stride, uint64_t* link_bar = nullptr) {
+                                        typename V2<R>::T* slot, int slot_stride) {
     int c[4];
     site_coords(g, par, (uint32_t)h, c);
     const int lex = lex_of(g, c);
@@ -759,17 +745,14 @@ __device__ __forceinline__ void hb_link(const Geom& g, const LinkField<R, NE>& U
     M3<R> u;
     if constexpr (SLOT) {
         const StapleSlot<R> S{slot, slot_stride}, Us{slot + 9 * slot_stride, slot_stride};
-        staple_rows_into<R, NE>(g, U, c, lex, par, MU, S);
-        KPDraws d = kp_draws_at(rng, 0u);
-        if (link_bar) {
-            // the block's own links were bulk-copied into the link slots while the staple was formed
-            if (!mbar_wait(link_bar, 0u, 1 << 20)) {
-                atomicOr(err, (int)DERR_BULK_WAIT);
-                return;  // link left unchanged; the host reports the error
-            }
-        } else {
-            Us.put(U.load(MU, par, h));
+        KPDraws d;
+        if constexpr (EARLY) {
+            d = kp_draws_at(rng, 0u);
+            cudaGridDependencySynchronize();
         }
+        staple_rows_into<R, NE, !EARLY>(g, U, c, lex, par, MU, S);
+        if constexpr (!EARLY) d = kp_draws_at(rng, 0u);
+        Us.put(U.load(MU, par, h));
         const int n_sub = 3 * n_hits;
 #pragma unroll 1
         for (int it = 0; it < n_sub; it++) {
@@ -798,39 +781,203 @@ struct HbSlotFits {
 };
 
 // Single-lattice heatbath launch: one thread per link of the (par, MU) set, geometry as kernel
-// parameters.
+// parameters.  Launched to follow the previous launch without a gap: the link's first draws need no link
+// and are formed before the wait for it.  The permission for the next launch is left to the blocks' ends
+// (given at their start or after the hits, the next launch's blocks crowd onto the SMs with room: a 16^4
+// sweep 252 and 181 us, at the ends 164).  A sweep at N_hits = 2: 12^4 148 to 133 us, 16^4 181 to 164, a
+// 131 k-site lattice 283 to 271; 24^4 and above 0-3%.
 template <typename R, int NE, int MU>
 __global__ void __launch_bounds__(QCB_HB_THREADS, QCB_HB_MINB(R))
     k_hb_subsweep(Geom g, LinkField<R, NE> U, int par, double c_alpha, int n_hits, uint64_t seed, uint32_t sweep,
                   int reproject, int* err) {
     static_assert(HbSlotFits<R, QCB_HB_THREADS>::value, "heatbath slot exceeds static shared memory");
     __shared__ typename V2<R>::T slot[18 * QCB_HB_THREADS];
-    uint64_t* link_bar = nullptr;
-#if QCB_HB_BULK_LINKS
-    // FP64 18-real: the block's own links U_mu(par, h) for its 128 half-sites are 4 whole 32-site
-    // tiles, element-major within a tile -- exactly the element-major layout of the link slots --
-    // so one thread bulk-copies them there (36 copies of 512 B; tiles past the field are skipped)
-    // and the copies land while the staple is formed.
-    __shared__ __align__(8) uint64_t bar;
-    if constexpr (sizeof(R) == 8 && NE == 9 && QCB_HB_THREADS == 128) {
-        if (threadIdx.x == 0) mbar_init(&bar, 1);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const int nT = (int)((g.Vh + 31) >> 5);
-            const int t0 = blockIdx.x * 4, t1 = min(t0 + 4, nT);
-            mbar_expect_tx(&bar, (unsigned)((t1 - t0) * 9 * 32 * sizeof(double2)));
-            for (int t = t0; t < t1; t++)
-                for (int e = 0; e < 9; e++)
-                    bulk_copy_g2s(slot + (9 + e) * 128 + (t - t0) * 32, U.p + U.tile0(MU, par, t * 32) + e * 32,
-                                  32 * sizeof(double2), &bar);
-        }
-        link_bar = &bar;
-    }
-#endif
     const int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= g.Vh) return;
-    hb_link<R, NE, MU, true>(g, U, par, (int)h, c_alpha, n_hits, seed, sweep, reproject, err, slot + threadIdx.x,
-                             QCB_HB_THREADS, link_bar);
+    hb_link<R, NE, MU, true, true>(g, U, par, (int)h, c_alpha, n_hits, seed, sweep, reproject, err,
+                                   slot + threadIdx.x, QCB_HB_THREADS);
+}
+
+// Heatbath sub-sweep of a small lattice (FP64): eight lanes a link, 16 links a block.  With one thread a
+// link, an 8^4 set is 64 warps on 148 SMs and a launch lasts as long as one link's serial chain (18 us:
+// three rounds of staple loads, then 6 subgroup updates of Philox calls, logarithms and a sine/cosine
+// each).  What does not depend on the updates in sequence is spread over the lanes:
+//   * the draws of the link's stream, whatever the attempts turn out to be: for every Philox call m its
+//     two uniforms, the attempt at m (log r1 + cos^2(2 pi r2) log r3 and delta^2, from calls m and
+//     m + 1) and the direction that call m would give (kp_fill).  They need no link, so they
+//     run before the wait for the previous launch and overlap its tail (with that and the
+//     permission to start given at the top, 83 to 68 us an 8^4 sweep);
+//   * the six staples, forward ones by warps 0-1 and backward ones by warps 2-3.
+// The updates run on the eight lanes alike, from registers.  Every value is formed by the operations of
+// k_hb_subsweep in their order: same links, bit for bit.  A sweep at N_hits = 2 (1): 4^4 44 (34) us
+// against 117 (81) with one thread a link, 8^4 68 (46) against 126 (87), 12^3 x 8 80 (54) against
+// 134 (95); past one wave of blocks (3 a SM: 7104 links) it is no faster (12^4 130 against 133, 16^4 353
+// against 164), which is where kHbGroupMaxVh lies.
+struct KPDraw {
+    double log_term, delta2;
+    KPDir dir;
+};
+constexpr int kHbLanes = 8, kHbGroupLinks = 16;
+constexpr int64_t kHbGroupMaxVh = 3 * 148 * kHbGroupLinks;
+constexpr int kKPTable = 24;  // stream positions held: 2 hits take 18 of them and 2 more a rejection
+static __device__ __noinline__ void kp_fill(uint64_t seed, uint32_t link, uint32_t sweep, uint32_t base, int count,
+                                     unsigned group, double2* raw, KPDraw* table) {
+    const LinkStream rng(seed, link, sweep, TAG_HB);
+    const int lane = threadIdx.x & (kHbLanes - 1);
+    __syncwarp(group);  // the old entries have been read
+    for (int m = lane; m < count; m += kHbLanes) raw[m] = rng.call(base + (uint32_t)m);
+    __syncwarp(group);
+    for (int m = lane; m < count; m += kHbLanes) {
+        const double2 P = raw[m];
+        KPDraw d;
+        d.dir = kp_direction(P);
+        d.log_term = 0.0;
+        if (m + 1 < count) {
+            const double2 Q = raw[m + 1];
+            d.log_term = kp_log(P.y, Q.x, Q.y);
+        }
+        d.delta2 = __dmul_rn(P.x, P.x);
+        table[m] = d;
+    }
+    __syncwarp(group);
+}
+template <int NE, int MU>
+__global__ void __launch_bounds__(kHbLanes* kHbGroupLinks)
+    k_hb_group(Geom g, LinkField<double, NE> U, int par, double c_alpha, int n_hits, uint64_t seed, uint32_t sweep,
+               int reproject, int* err) {
+    __shared__ KPDraw table_s[kHbGroupLinks][kKPTable];
+    __shared__ double2 raw_s[kHbGroupLinks][kKPTable];
+    __shared__ double2 part[6][9][kHbGroupLinks], sum[kHbGroupLinks][9];
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int slot = threadIdx.x / kHbLanes;
+    const unsigned group = 0xffu << (threadIdx.x & 24);
+    // links past the set repeat its last one and store nothing
+    const int64_t h0 = (int64_t)blockIdx.x * kHbGroupLinks, last = g.Vh - 1;
+    const bool live = h0 + slot <= last;
+    const int h = (int)(live ? h0 + slot : last);
+    int c[4];
+    site_coords(g, par, (uint32_t)h, c);
+    const uint32_t link = (uint32_t)lex_of(g, c) * 4u + (uint32_t)MU;
+    KPDraw* table = table_s[slot];
+    // the subgroups' calls and room for three rejections
+    int held = n_hits < 2 ? 9 * n_hits + 6 : kKPTable;
+    kp_fill(seed, link, sweep, 0u, held, group, raw_s[slot], table);
+    cudaGridDependencySynchronize();
+    {
+        // staple task: link (threadIdx & 15), k-th nu, in the order of staple_rows_into
+        const int i = threadIdx.x & 63, k = i >> 4;
+        const bool fwd = threadIdx.x < 64;
+        if (k < 3) {
+            const int hl = (int)(h0 + (i & 15) <= last ? h0 + (i & 15) : last);
+            int cl[4];
+            site_coords(g, par, (uint32_t)hl, cl);
+            const int lex = lex_of(g, cl), opp = par ^ 1;
+            const Steps st = make_steps(g, cl);
+            const int nu = k < MU ? k : k + 1;
+            const int xmu = lex + st.up[MU], dnu = sel4(st.dn, nu), xmnu = lex + dnu;
+            Cx<double> r[2][3];
+            if (fwd) {
+                const M3<double> a = U.load(nu, opp, xmu >> 1);
+                const M3<double> b = U.load(MU, opp, (lex + sel4(st.up, nu)) >> 1);
+                const M3<double> d = U.load(nu, par, lex >> 1);
+                Cx<double> t[2][3];
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        t[i][j] = mkc<double>(0, 0);
+#pragma unroll
+                        for (int q = 0; q < 3; q++) cmac_nc(t[i][j], a(i, q), b(j, q));
+                    }
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        r[i][j] = mkc<double>(0, 0);
+#pragma unroll
+                        for (int q = 0; q < 3; q++) cmac_nc(r[i][j], t[i][q], d(j, q));
+                    }
+            } else {
+                const M3<double> v1 = U.load(MU, opp, xmnu >> 1);
+                const M3<double> v0 = U.load(nu, par, (xmu + dnu) >> 1);
+                const M3<double> v2 = U.load(nu, opp, xmnu >> 1);
+                Cx<double> t[3][2];
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        t[i][j] = mkc<double>(0, 0);
+#pragma unroll
+                        for (int q = 0; q < 3; q++) cmac(t[i][j], v1(i, q), v0(q, j));
+                    }
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        r[i][j] = mkc<double>(0, 0);
+#pragma unroll
+                        for (int q = 0; q < 3; q++) cmac_cn(r[i][j], t[q][i], v2(q, j));
+                    }
+            }
+            double2(*p)[kHbGroupLinks] = part[2 * k + (fwd ? 0 : 1)];
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const int j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+                const Cx<double> r2 = conj_cross(r[0][j1], r[1][j2], r[0][j2], r[1][j1]);
+                p[j][i & 15] = make_double2(r[0][j].re, r[0][j].im);
+                p[3 + j][i & 15] = make_double2(r[1][j].re, r[1][j].im);
+                p[6 + j][i & 15] = make_double2(r2.re, r2.im);
+            }
+        }
+    }
+    M3<double> u = U.load(MU, par, h);
+    __syncthreads();
+    for (int t = threadIdx.x; t < 9 * kHbGroupLinks; t += kHbLanes * kHbGroupLinks) {
+        const int e = t >> 4, l = t & 15;
+        double2 v = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int s = 0; s < 6; s++) {
+            v.x += part[s][e][l].x;
+            v.y += part[s][e][l].y;
+        }
+        sum[l][e] = v;
+    }
+    __syncthreads();
+    M3<double> A;
+#pragma unroll
+    for (int e = 0; e < 9; e++) A.e[e] = mkc<double>(sum[slot][e].x, sum[slot][e].y);
+    uint32_t base = 0, n = 0;  // position of table[0], position of the next attempt
+    // su2_step with its draws from the table
+    auto step = [&](const Quat& w) {
+        const double ik = rsqrt(w.a0 * w.a0 + w.a1 * w.a1 + w.a2 * w.a2 + w.a3 * w.a3);
+        const Quat v = {w.a0 * ik, w.a1 * ik, w.a2 * ik, w.a3 * ik};
+        const double m05a = c_alpha * ik;
+        const int cap = (m05a < 0.0 && isfinite(m05a)) ? KP_MAX_ATTEMPTS : 0;
+        for (int it = 0; it < cap; it++) {
+            if ((int)(n - base) > held - 3) {
+                kp_fill(seed, link, sweep, n, kKPTable, group, raw_s[slot], table);
+                base = n;
+                held = kKPTable;
+            }
+            const KPDraw* d = table + (n - base);
+            const double lsq = __dmul_rn(m05a, d->log_term);
+            if (d->delta2 <= __dadd_rn(1.0, -lsq)) {
+                n += 3u;
+                return kp_element(__dadd_rn(1.0, -__dmul_rn(2.0, lsq)), d[2].dir, v);
+            }
+            n += 2u;
+        }
+        if ((threadIdx.x & (kHbLanes - 1)) == 0) atomicOr(err, cap > 0 ? (int)DERR_KP_CAP : (int)DERR_KP_SCALE);
+        return Quat{1.0, 0.0, 0.0, 0.0};
+    };
+#pragma unroll 1
+    for (int hit = 0; hit < n_hits; hit++) {
+        cm_apply<double, 0, 1>(u, step(cm_quaternion<double, 0, 1>(u, A)));
+        cm_apply<double, 1, 2>(u, step(cm_quaternion<double, 1, 2>(u, A)));
+        cm_apply<double, 0, 2>(u, step(cm_quaternion<double, 0, 2>(u, A)));
+    }
+    if (reproject) reproject_fp64(u);
+    if (live && (threadIdx.x & (kHbLanes - 1)) == 0) U.store(MU, par, h, u);
 }
 
 // One link's heatbath update (the C ABI's single-link entry, qcb_hb_link; reference
