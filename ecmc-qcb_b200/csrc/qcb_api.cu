@@ -155,10 +155,9 @@ int check_err_flag(qcb_field_s* f) {
 }
 
 // reduction of nb partial vectors of nv doubles into dst (device)
-int finalize(qcb_field_s* f, int nb, int nv, unsigned max_mask, double* dst) {
+int finalize(qcb_field_s* f, int nb, int nv, unsigned max_mask, double* dst, int* row = nullptr) {
     return launch(f, QCB_K_OTHER, [&] {
-        k_finalize<<<1, 256, 0, f->stream>>>(f->partials, nb, nv, max_mask, dst);
-        return cudaGetLastError();
+        return launch_early(k_finalize, 1, kFinalizeThreads * nv, f->stream, f->partials, nb, nv, max_mask, dst, row);
     });
 }
 
@@ -173,11 +172,11 @@ int enq_plaquette(qcb_field_s* f, double* dst) {
 // One block per 128 half-sites (up to the grid's y limit): the blocks run in site order, so the
 // pass sweeps the lattice once in t and a link's neighbours are still in L2 when the front reaches
 // them (a capped grid-stride loop jumps across the lattice and re-reads them from DRAM).
-int enq_clover(qcb_field_s* f, double* dst) {
+int enq_clover(qcb_field_s* f, double* dst, int* row = nullptr) {
     const unsigned nbx = clover_blocks(f->g.Vh);
     RET(ensure_partials(f, (size_t)nbx * 6 * 3));
     RET(launch(f, QCB_K_CLOVER, [&] { return fmt_ops(f->fmt).clover(f->g, f->links, f->partials, nbx, f->stream); }));
-    return finalize(f, (int)(nbx * 6), 3, 0u, dst);
+    return finalize(f, (int)(nbx * 6), 3, 0u, dst, row);
 }
 
 int read_results(qcb_field_s* f, int n) {
@@ -215,10 +214,10 @@ int flow_step(qcb_flow_s* fl) {
 
 // One RK3 step that also measures its input configuration: stage 1 writes the clover halves
 // (k_flow_stage1_meas; its links are those of the plain stage 1), their per-site sum gives
-// (q, e, plaquette sum) in dst[0..2], then stages 2 and 3 as in flow_step.  The standalone clover
+// (q, e, plaquette sum) in the next row of the measurements, then stages 2 and 3 as in flow_step.  The standalone clover
 // pass forms every leaf with three products a plane and site; here the force's own staples give
 // the clover with two products a plane and link.
-int flow_step_meas(qcb_flow_s* fl, double* dst) {
+int flow_step_meas(qcb_flow_s* fl) {
     qcb_field_s* f = fl->fld;
     RET(ensure_alt(f));
     const int rep = needs_reproject(f->prec, f->store);
@@ -228,7 +227,7 @@ int flow_step_meas(qcb_flow_s* fl, double* dst) {
     const unsigned nb = halves_blocks(f->g.Vh);
     RET(launch(f, QCB_K_CLOVER,
                [&] { return fmt_ops(f->fmt).clover_halves(f->g, fl->halves, f->partials, nb, f->stream); }));
-    RET(finalize(f, (int)nb, 3, 0u, dst));
+    RET(finalize(f, (int)nb, 3, 0u, fl->d_meas, fl->d_count));
     for (int stage = 2; stage <= 3; stage++) {
         void* win = (stage == 2) ? f->alt : f->links;
         void* wout = (stage == 2) ? f->links : f->alt;
@@ -244,7 +243,7 @@ int flow_step_meas(qcb_flow_s* fl, double* dst) {
 // The measurement of the flowed field alone through the measuring stage 1 (its stage-1 output, in
 // the spare buffer, is left unused): the last measurement of a run, so that every row of a measured
 // flow comes from the same arithmetic.
-int meas_halves_only(qcb_flow_s* fl, double* dst) {
+int meas_halves_only(qcb_flow_s* fl) {
     qcb_field_s* f = fl->fld;
     RET(ensure_alt(f));
     const int rep = needs_reproject(f->prec, f->store);
@@ -254,19 +253,16 @@ int meas_halves_only(qcb_flow_s* fl, double* dst) {
     const unsigned nb = halves_blocks(f->g.Vh);
     RET(launch(f, QCB_K_CLOVER,
                [&] { return fmt_ops(f->fmt).clover_halves(f->g, fl->halves, f->partials, nb, f->stream); }));
-    return finalize(f, (int)nb, 3, 0u, dst);
+    return finalize(f, (int)nb, 3, 0u, fl->d_meas, fl->d_count);
 }
 
 // ------------------------------------------------------------------ flow step graphs
 // Without per-launch timing, the flow's repeated launch sequences are captured once as CUDA graphs
 // and replayed: two RK3 steps (six stage launches; the ping-pong buffers are back in place after
-// them), and one measurement block of qcb_flow_measure (clover pass into a fixed slot, the row
-// scatter, then n_rk RK3 steps).  Replays launch the same kernels with the same arguments as the
+// them), and one measurement block of qcb_flow_measure (the measurement into the next row, then
+// n_rk RK3 steps).  Replays launch the same kernels with the same arguments as the
 // plain launches, so results are identical bit for bit.
-constexpr int kMeasSlot = 32;  // d_res offset of the measurement slot (q, e, plaquette sums)
-
 int meas_block(qcb_flow_s* fl, int n_rk);
-__global__ void k_meas_scatter(const double* slot, double* meas, int* counter);
 // Graphs need a capturable stream: not the legacy default stream, and no per-launch timing events.
 bool graphs_ok(const qcb_field_s* f) { return !f->timing && f->stream != nullptr; }
 
@@ -341,24 +337,19 @@ int flow_graph_run(qcb_flow_s* fl, int kind, int n_rk) {
     return QCB_OK;
 }
 
-// One measurement of the flowed field -- (q, e and the plaquette sum) into the fixed slot, copied to
-// the next row of the measurement buffer -- followed by n_rk RK3 steps.  With the halves buffer in
+// One measurement of the flowed field -- q, e and the plaquette sum into the next row of the
+// measurement buffer -- followed by n_rk RK3 steps.  With the halves buffer in
 // place (measured flows with RK3 steps) the measurement comes from the measuring stage 1: that of
 // the following step, or for the last measurement one whose output is left unused.
 int meas_block(qcb_flow_s* fl, int n_rk) {
     qcb_field_s* f = fl->fld;
-    double* slot = f->d_res + kMeasSlot;
     const bool fused = n_rk > 0 && fl->halves;
     if (fused)
-        RET(flow_step_meas(fl, slot));
+        RET(flow_step_meas(fl));
     else if (fl->halves)
-        RET(meas_halves_only(fl, slot));
+        RET(meas_halves_only(fl));
     else
-        RET(enq_clover(f, slot));
-    RET(launch(f, QCB_K_OTHER, [&] {
-        k_meas_scatter<<<1, 1, 0, f->stream>>>(slot, fl->d_meas, fl->d_count);
-        return cudaGetLastError();
-    }));
+        RET(enq_clover(f, fl->d_meas, fl->d_count));
     for (int k = fused ? 1 : 0; k < n_rk; k++) RET(flow_step(fl));
     return QCB_OK;
 }
@@ -415,24 +406,29 @@ int field_new(const int L[4], int prec, int store, cudaStream_t stream, qcb_fiel
 }  // namespace
 
 // Deterministic final reduction (one block, fixed summation order for a given nb).
-__global__ void qcb::k_finalize(const double* partials, int nb, int nv, unsigned max_mask, double* out) {
-    __shared__ double sm[256];
-    for (int k = 0; k < nv; k++) {
-        const bool ismax = (max_mask >> k) & 1u;
-        double acc = 0.0;
-        for (int i = threadIdx.x; i < nb; i += 256) {
-            double v = partials[(size_t)i * nv + k];
-            acc = ismax ? fmax(acc, v) : acc + v;
-        }
-        sm[threadIdx.x] = acc;
+__global__ void qcb::k_finalize(const double* __restrict__ partials, int nb, int nv, unsigned max_mask, double* out,
+                                int* row) {
+    __shared__ double sm[4 * kFinalizeThreads];
+    const int k = threadIdx.x / kFinalizeThreads, t = threadIdx.x % kFinalizeThreads;
+    const bool ismax = (max_mask >> k) & 1u;
+    cudaGridDependencySynchronize();
+    double acc = 0.0;
+#pragma unroll 4
+    for (int i = t; i < nb; i += kFinalizeThreads) {
+        const double v = partials[(size_t)i * nv + k];
+        acc = ismax ? fmax(acc, v) : acc + v;
+    }
+    double* s = sm + k * kFinalizeThreads;
+    s[t] = acc;
+    __syncthreads();
+    for (int w = kFinalizeThreads / 2; w > 0; w >>= 1) {
+        if (t < w) s[t] = ismax ? fmax(s[t], s[t + w]) : s[t] + s[t + w];
         __syncthreads();
-        for (int s = 128; s > 0; s >>= 1) {
-            if ((int)threadIdx.x < s) sm[threadIdx.x] = ismax ? fmax(sm[threadIdx.x], sm[threadIdx.x + s])
-                                                              : sm[threadIdx.x] + sm[threadIdx.x + s];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[k] = sm[0];
+    }
+    if (t == 0) out[(row ? (size_t)*row * nv : 0) + k] = s[0];
+    if (row) {
         __syncthreads();
+        if (threadIdx.x == 0) *row += 1;
     }
 }
 
@@ -495,16 +491,6 @@ __global__ void __launch_bounds__(256) k_fma_rate(T a, T b, int iters, T* out) {
     if (s == (T)-1) out[0] = s;  // never true for these inputs; keeps the chains
 }
 
-// Copies one measurement (q, e, plaquette sums) from the fixed slot the clover pass wrote into row
-// *counter of the measurement buffer and advances the counter (one thread; the host sizes the buffer
-// for every row it launches).
-__global__ void k_meas_scatter(const double* slot, double* meas, int* counter) {
-    const int c = *counter;
-    meas[3 * c] = slot[0];
-    meas[3 * c + 1] = slot[1];
-    meas[3 * c + 2] = slot[2];
-    *counter = c + 1;
-}
 __global__ void k_diag_philox(uint4 ctr, uint2 key, int n, uint4* out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;

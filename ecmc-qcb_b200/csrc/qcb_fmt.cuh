@@ -28,23 +28,6 @@ struct FmtImpl {
         return *cache;
     }
 
-    // Launch of a kernel that begins with work of its own and then waits for the launches before it
-    // (cudaGridDependencySynchronize): its blocks may start when those of the previous launch have
-    // ended or have said that they may, without the gap between two launches in a stream.
-    template <typename... P, typename... A>
-    static cudaError_t launch_early(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, A... a) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(block);
-        cfg.stream = s;
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
-    }
-
     template <int MU, int BLOCK, int MINB>
     static cudaError_t hb_launch(const WorkList& w, int par, int n_hits, const uint32_t* sweep_dev, uint32_t sweep_add,
                                  int reproject, int* err, cudaStream_t s) {
@@ -133,13 +116,8 @@ struct FmtImpl {
         AlgField<R> za;
         za.p = (typename AlgField<R>::C2*)z;
         za.Vh = g.Vh;
-        if (stage == 1)
-            k_flow_stage<R, NE, 1><<<nb, QCB_FLOW_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps, rep);
-        else if (stage == 2)
-            k_flow_stage<R, NE, 2><<<nb, QCB_FLOW_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps, rep);
-        else
-            k_flow_stage<R, NE, 3><<<nb, QCB_FLOW_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps, rep);
-        return cudaGetLastError();
+        const auto k = stage == 1 ? k_flow_stage<R, NE, 1> : (stage == 2 ? k_flow_stage<R, NE, 2> : k_flow_stage<R, NE, 3>);
+        return launch_early(k, nb, QCB_FLOW_THREADS, s, g, view(win, g.Vh), view(wout, g.Vh), za, eps, rep);
     }
 
     static cudaError_t flow1_meas(const Geom& g, const void* win, void* wout, void* z, double eps, int rep,
@@ -149,14 +127,12 @@ struct FmtImpl {
         za.p = (typename AlgField<R>::C2*)z;
         za.Vh = g.Vh;
         const HalfClovers<R> H{(R*)hbuf, 2 * g.Vh};
-        k_flow_stage1_meas<R, NE><<<nb, QCB_FLOW_THREADS, 0, s>>>(g, view(win, g.Vh), view(wout, g.Vh), za, eps,
-                                                                   rep, H);
-        return cudaGetLastError();
+        return launch_early(k_flow_stage1_meas<R, NE>, nb, QCB_FLOW_THREADS, s, g, view(win, g.Vh), view(wout, g.Vh), za,
+                            eps, rep, H);
     }
     static cudaError_t clover_halves(const Geom& g, const void* hbuf, double* partials, unsigned nb, cudaStream_t s) {
         const HalfClovers<R> H{(R*)hbuf, 2 * g.Vh};
-        k_clover_halves<R><<<nb, 128, 0, s>>>(g, H, partials);
-        return cudaGetLastError();
+        return launch_early(k_clover_halves<R>, nb, 128, s, g, H, partials);
     }
 
     static AlgField<R> alg(const void* p, int64_t Vh) {

@@ -103,7 +103,7 @@ __device__ __forceinline__ M3<R> staple_rt(const Geom& g, const LinkField<R, NE>
 // links' distance from SU(3), which in FP32 storage is the FP32 rounding level (~1e-7).
 // FLOW: the FP64 flow kernels' order of nu, mu ^ 1, mu ^ 2, mu ^ 3, in which the warps of mu and nu are in
 // the same plane at the same time and share its links in L1; else ascending, as compute_staple.
-template <typename R, int NE, bool FLOW = false>
+template <typename R, int NE, bool FLOW = false, bool EARLY = false>
 __device__ __forceinline__ M3<R> staple_rt_rows(const Geom& g, const LinkField<R, NE>& U, const int c[4],
                                                 int lex, int par, int mu) {
     M3<R> A;
@@ -119,8 +119,8 @@ __device__ __forceinline__ M3<R> staple_rt_rows(const Geom& g, const LinkField<R
         const int xmnu = lex + dnu;
         const int xmumnu = xmu + dnu;  // x+mu has the same nu coordinate as x
         {
-            const M3<R> a = U.load_ro(nu, opp, xmu >> 1);
-            const M3<R> b = U.load_ro(mu, opp, xnu >> 1);
+            const M3<R> a = U.template load_t<!EARLY>(nu, opp, xmu >> 1);
+            const M3<R> b = U.template load_t<!EARLY>(mu, opp, xnu >> 1);
             Cx<R> t[2][3], s[2][3];
 #pragma unroll
             for (int i = 0; i < 2; i++)
@@ -130,7 +130,7 @@ __device__ __forceinline__ M3<R> staple_rt_rows(const Geom& g, const LinkField<R
 #pragma unroll
                     for (int q = 0; q < 3; q++) cmac_nc(t[i][j], a(i, q), b(j, q));
                 }
-            const M3<R> d = U.load_ro(nu, par, lex >> 1);
+            const M3<R> d = U.template load_t<!EARLY>(nu, par, lex >> 1);
 #pragma unroll
             for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -147,8 +147,8 @@ __device__ __forceinline__ M3<R> staple_rt_rows(const Geom& g, const LinkField<R
             }
         }
         {
-            const M3<R> v1 = U.load_ro(mu, opp, xmnu >> 1);
-            const M3<R> v0 = U.load_ro(nu, par, xmumnu >> 1);
+            const M3<R> v1 = U.template load_t<!EARLY>(mu, opp, xmnu >> 1);
+            const M3<R> v0 = U.template load_t<!EARLY>(nu, par, xmumnu >> 1);
             Cx<R> t[3][2], s[2][3];
 #pragma unroll
             for (int i = 0; i < 3; i++)
@@ -158,7 +158,7 @@ __device__ __forceinline__ M3<R> staple_rt_rows(const Geom& g, const LinkField<R
 #pragma unroll
                     for (int q = 0; q < 3; q++) cmac(t[i][j], v1(i, q), v0(q, j));
                 }
-            const M3<R> v2 = U.load_ro(nu, opp, xmnu >> 1);
+            const M3<R> v2 = U.template load_t<!EARLY>(nu, opp, xmnu >> 1);
 #pragma unroll
             for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -258,7 +258,7 @@ __device__ __forceinline__ void acc_product(const M3<R>& A, const M3<R>& B, R ou
 
 // staple_rt_rows, and for the planes this direction handles the two clover halves and the plaquette
 // trace of the link's site (see above).  u is the link U_mu(x) itself.
-template <typename R, int NE>
+template <typename R, int NE, bool EARLY>
 __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkField<R, NE>& U, const int c[4],
                                                      int lex, int par, int mu, const M3<R>& u_in,
                                                      const HalfClovers<R>& H) {
@@ -279,8 +279,8 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
         const int xmumnu = xmu + dnu;
         M3<R> Sf;
         {
-            const M3<R> a = U.load_ro(nu, opp, xmu >> 1);
-            const M3<R> b = U.load_ro(mu, opp, xnu >> 1);
+            const M3<R> a = U.template load_t<!EARLY>(nu, opp, xmu >> 1);
+            const M3<R> b = U.template load_t<!EARLY>(mu, opp, xnu >> 1);
             Cx<R> t[2][3];
 #pragma unroll
             for (int i = 0; i < 2; i++)
@@ -290,7 +290,7 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
 #pragma unroll
                     for (int q = 0; q < 3; q++) cmac_nc(t[i][j], a(i, q), b(j, q));
                 }
-            const M3<R> d = U.load_ro(nu, par, lex >> 1);
+            const M3<R> d = U.template load_t<!EARLY>(nu, par, lex >> 1);
 #pragma unroll
             for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -310,8 +310,8 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
         }
         M3<R> Sb;
         {
-            const M3<R> v1 = U.load_ro(mu, opp, xmnu >> 1);
-            const M3<R> v0 = U.load_ro(nu, par, xmumnu >> 1);
+            const M3<R> v1 = U.template load_t<!EARLY>(mu, opp, xmnu >> 1);
+            const M3<R> v0 = U.template load_t<!EARLY>(nu, par, xmumnu >> 1);
             Cx<R> t[3][2];
 #pragma unroll
             for (int i = 0; i < 3; i++)
@@ -321,7 +321,7 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
 #pragma unroll
                     for (int q = 0; q < 3; q++) cmac(t[i][j], v1(i, q), v0(q, j));
                 }
-            const M3<R> v2 = U.load_ro(nu, opp, xmnu >> 1);
+            const M3<R> v2 = U.template load_t<!EARLY>(nu, opp, xmnu >> 1);
 #pragma unroll
             for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -343,7 +343,7 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
             // FP64: the link is reloaded here (an L1 hit) instead of held across the loop, which
             // lets the kernel run 3 blocks/SM (measured flow 2.73-2.74 against 2.79-2.80 ms a 32^4
             // step); FP32 holds it (no gain from the reload)
-            const M3<R> u = (sizeof(R) == 8) ? U.load_ro(mu, par, lex >> 1) : u_in;
+            const M3<R> u = (sizeof(R) == 8) ? U.template load_t<!EARLY>(mu, par, lex >> 1) : u_in;
             R tr = R(0);
 #pragma unroll
             for (int i = 0; i < 3; i++)
@@ -1005,7 +1005,7 @@ __global__ void k_hb_one(Geom g, LinkField<R, NE> U, int par, int h, double c_al
 //   stage 3: W' = exp(3/4 eps F - eps Z) W                          compute_w3
 // The whole field of forces is never materialised: Win is read-only for the launch and W'
 // goes to a second buffer (ping-pong), which is what makes force and update one pass.
-template <typename R, int NE, int STAGE, bool MEAS = false>
+template <typename R, int NE, int STAGE, bool MEAS = false, bool EARLY = false>
 __device__ __forceinline__ void flow_link(const Geom& g, const LinkField<R, NE>& Win, const LinkField<R, NE>& Wout,
                                           const AlgField<R>& Z, double eps, int mu, int par, int h,
                                           int reproject, const HalfClovers<R>& H = HalfClovers<R>{}) {
@@ -1013,23 +1013,24 @@ __device__ __forceinline__ void flow_link(const Geom& g, const LinkField<R, NE>&
     int c[4];
     site_coords(g, par, (uint32_t)h, c);
     const int lex = lex_of(g, c);
+    if constexpr (EARLY) cudaGridDependencySynchronize();
     AntiH<R> F;
     M3<R> u;
     if constexpr (MEAS) {
         // the same staple and force, with the clover halves of the input configuration
         if constexpr (sizeof(R) == 8) {  // the link reloaded where the halves need it
-            const M3<R> A = staple_rt_rows_meas<R, NE>(g, Win, c, lex, par, mu, u, H);
-            u = Win.load_ro(mu, par, h);
+            const M3<R> A = staple_rt_rows_meas<R, NE, EARLY>(g, Win, c, lex, par, mu, u, H);
+            u = Win.template load_t<!EARLY>(mu, par, h);
             F = neg_proj_lie_mul(u, A);
         } else {
-            u = Win.load_ro(mu, par, h);
-            const M3<R> A = staple_rt_rows_meas<R, NE>(g, Win, c, lex, par, mu, u, H);
+            u = Win.template load_t<!EARLY>(mu, par, h);
+            const M3<R> A = staple_rt_rows_meas<R, NE, EARLY>(g, Win, c, lex, par, mu, u, H);
             F = neg_proj_lie_mul(u, A);
         }
     } else {
         // two-row staple products and the projection's entries only
-        const M3<R> A = staple_rt_rows<R, NE, sizeof(R) == 8>(g, Win, c, lex, par, mu);
-        u = Win.load_ro(mu, par, h);
+        const M3<R> A = staple_rt_rows<R, NE, sizeof(R) == 8, EARLY>(g, Win, c, lex, par, mu);
+        u = Win.template load_t<!EARLY>(mu, par, h);
         F = neg_proj_lie_mul(u, A);
     }
     AntiH<R> X;
@@ -1080,7 +1081,7 @@ __global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW1_MINB(R))
     int64_t h;
     flow_map<R>(blockIdx.x, mu, par, h);
     if (h >= g.Vh) return;
-    flow_link<R, NE, STAGE>(g, Win, Wout, Z, eps, mu, par, (int)h, reproject);
+    flow_link<R, NE, STAGE, false, true>(g, Win, Wout, Z, eps, mu, par, (int)h, reproject);
 }
 
 // Stage 1 that also writes the clover halves of its input configuration (the measurement of a
@@ -1094,7 +1095,7 @@ __global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MEAS_MINB(R))
     int64_t h;
     flow_map<R>(blockIdx.x, mu, par, h);
     if (h >= g.Vh) return;
-    flow_link<R, NE, 1, true>(g, Win, Wout, Z, eps, mu, par, (int)h, reproject, H);
+    flow_link<R, NE, 1, true, true>(g, Win, Wout, Z, eps, mu, par, (int)h, reproject, H);
 }
 
 // ------------------------------------------------------------------ the reference's separate flow passes
@@ -1173,9 +1174,12 @@ __device__ __forceinline__ void block_sum_store(double v[NV], double* partials, 
     }
 }
 
-// Deterministic final sum of nb partial vectors (one block of 256 threads; fixed order).
-// mode bit k set: component k is a max instead of a sum.
-__global__ void k_finalize(const double* partials, int nb, int nv, unsigned max_mask, double* out);
+// Deterministic final sum of nb partial vectors of nv components (one block of 256 threads a component;
+// fixed order).  Bit k of max_mask set: component k is a max instead of a sum.  Into out[0..nv), or
+// with a row counter into row *row of out, which then advances.
+constexpr int kFinalizeThreads = 256;
+__global__ void k_finalize(const double* __restrict__ partials, int nb, int nv, unsigned max_mask, double* out,
+                           int* row);
 
 // Plaquette (observables_mpi.cpp:11-35): per site sum over mu<nu of Re Tr(U_mu(x) U_nu(x+mu)
 // U_mu(x+nu)^dag U_nu(x)^dag)/3, evaluated as Re Tr((U_mu(x) U_nu(x+mu)) (U_nu(x) U_mu(x+nu))^dag).
@@ -1480,6 +1484,7 @@ template <typename R>
 __global__ void __launch_bounds__(128) k_clover_halves(Geom g, HalfClovers<R> H, double* partials) {
     double v[3] = {0.0, 0.0, 0.0};
     const int64_t site = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    cudaGridDependencySynchronize();
     if (site < H.V) site_halves_qe(H, site, v);
     block_sum_store<3>(v, partials, blockIdx.x);
 }

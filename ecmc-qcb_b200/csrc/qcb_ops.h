@@ -10,6 +10,23 @@
 
 namespace qcb {
 
+// Launch of a kernel that begins with work of its own and then waits for the launches before it
+// (cudaGridDependencySynchronize): its blocks may start when those of the previous launch have
+// ended or have said that they may, without the gap between two launches in a stream.
+template <typename... P, typename... A>
+inline cudaError_t launch_early(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, A... a) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
+}
+
 // A work list of tiles over device-resident lattice descriptors.
 struct WorkList {
     const LatDesc* lats = nullptr;  // device array of nlat descriptors; NULL: use `one`

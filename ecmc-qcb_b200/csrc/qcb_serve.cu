@@ -291,7 +291,7 @@ bool measure_big(qcb_server_s* s, Request* r, int flip_xor) {
                  "clover launch"))
         return false;
     double* slot = (double*)((char*)r->buf + r->off_meas) + (size_t)(s->tick_b - r->tick0) * 3;
-    k_finalize<<<1, 256, 0, s->stream>>>(s->big_partials, (int)(nbx * 6), 3, 0u, slot);
+    k_finalize<<<1, 3 * kFinalizeThreads, 0, s->stream>>>(s->big_partials, (int)(nbx * 6), 3, 0u, slot, nullptr);
     note_launches(2);
     return cuda_ok(s, cudaGetLastError(), "measure finalize");
 }
@@ -312,7 +312,7 @@ bool flow_big_meas(qcb_server_s* s, Request* r, int flip_xor, int rep) {
                  "flow launch"))
         return false;
     if (!cuda_ok(s, o.clover_halves(r->g, s->halves, s->big_partials, nb, s->stream), "clover launch")) return false;
-    k_finalize<<<1, 256, 0, s->stream>>>(s->big_partials, (int)nb, 3, 0u, r->meas_slot);
+    k_finalize<<<1, 3 * kFinalizeThreads, 0, s->stream>>>(s->big_partials, (int)nb, 3, 0u, r->meas_slot, nullptr);
     note_launches(3);
     r->meas_slot = nullptr;
     return cuda_ok(s, cudaGetLastError(), "measure finalize");

@@ -272,11 +272,14 @@ QCB_HD void ch_horner(double t, double d, double q[6]) {
     q[4] = q2r;
     q[5] = q2i;
 }
-// The reference's 18 terms, or 11 where they give the same double: the eigenvalues of X obey
-// |l|^2 <= 4t/3, so for t <= 1/32 the terms from n = 12 on add up to less than
-// (1/24)^6 / 12! = 1.1e-17 of the result.
+// The reference's 18 terms; for FP64 matrices 11 where they give the same sum: the eigenvalues of X obey
+// |l|^2 <= 4t/3, so for t <= 1/32 the terms from n = 12 on add up to less than (1/24)^6 / 12! = 1.1e-17
+// of the result.  FP32 matrices keep 18: the imaginary parts are small, so the dropped terms would
+// now and then round them to another float, and one such link makes the whole flowed field round
+// differently.
+template <typename R>
 QCB_HD void ch_coeffs(double t, double d, double q[6]) {
-    if (t <= 0.03125)
+    if (sizeof(R) == 8 && t <= 0.03125)
         ch_horner<11>(t, d, q);
     else
         ch_horner<18>(t, d, q);
@@ -308,7 +311,7 @@ QCB_HD M3<R> exp_su3(const AntiH<R>& X) {
         d = fma(a0 * a1, a2, fma(2.0, im3, -fma(a0, n12, fma(a1, n02, a2 * n01))));
     }
     double q[6];
-    ch_coeffs(t, d, q);
+    ch_coeffs<R>(t, d, q);
     const Cx<R> q0 = mkc<R>((R)q[0], (R)q[1]), q1 = mkc<R>((R)q[2], (R)q[3]), q2 = mkc<R>((R)q[4], (R)q[5]);
     // -|z|^2 added to r
     auto sub_norm = [](Cx<R> z, R r) { return fma(-z.re, z.re, fma(-z.im, z.im, r)); };
@@ -325,7 +328,7 @@ QCB_HD M3<R> exp_su3(const AntiH<R>& X) {
     x2[1].re = fma(-o[1].im, a[2], x2[1].re);
     x2[1].im = fma(o[1].re, a[2], x2[1].im);
     x2[2].re = fma(-o[0].re, o[1].re, -(o[0].im * o[1].im));
-    x2[2].im = fma(-o[0].re, o[1].im, o[0].im * o[1].re);
+    x2[2].im = fma(o[0].im, o[1].re, -(o[0].re * o[1].im));
     x2[2].re = fma(-o[2].im, a[2], fma(-a[1], o[2].im, x2[2].re));
     x2[2].im = fma(o[2].re, a[2], fma(a[1], o[2].re, x2[2].im));
     M3<R> E;
