@@ -692,11 +692,12 @@ int qcb_field_copy(qcb_field dst, qcb_field src) {
         CK(cudaMemcpyAsync(dst->links, src->links, link_bytes(dst->fmt, dst->g.Vh), cudaMemcpyDeviceToDevice,
                            dst->stream));
     } else {
-        RET(staging_acquire(dst));
-        RET(launch(dst, QCB_K_OTHER,
-                   [&] { return fmt_ops(src->fmt).soa_to_aos(src->g, src->links, dst->staging, 0, dst->stream); }));
-        RET(upload_from_staging(dst, 0));
-        RET(staging_release(dst));
+        // (refused while a prefetched configuration waits, as every change of the links but its commit)
+        if (dst->prefetch_pending)
+            return fail(QCB_EINVAL, "a prefetched configuration occupies the staging buffer: commit it first");
+        RET(launch(dst, QCB_K_OTHER, [&] {
+            return fmt_ops(dst->fmt).convert_links(dst->g, src->fmt, src->links, dst->links, dst->stream);
+        }));
     }
     // src's later work (a heatbath, an upload) must not overwrite src's links while dst's stream is
     // still reading them: src's stream waits for the end of the copy.

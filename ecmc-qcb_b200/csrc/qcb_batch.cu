@@ -148,12 +148,9 @@ int capture(qcb_batch_s* b, int n_hits, int variant) {
 
 // Copies every lattice of b into dst (same lattices, possibly another storage format).
 int convert_into(qcb_batch_s* b, qcb_batch_s* dst) {
-    if (!b->staging) CK(cudaMalloc(&b->staging, (size_t)b->max_V * 36 * sizeof(double2)));
-    for (int i = 0; i < b->n; i++) {
-        CK(fmt_ops(b->fmt).soa_to_aos(b->desc[i].g, b->desc[i].links, b->staging, 0, b->stream));
-        CK(fmt_ops(dst->fmt).aos_to_soa(dst->desc[i].g, b->staging, dst->desc[i].links, 0, b->stream));
-    }
-    note_launches(2 * b->n);
+    for (int i = 0; i < b->n; i++)
+        CK(fmt_ops(dst->fmt).convert_links(b->desc[i].g, b->fmt, b->desc[i].links, dst->desc[i].links, b->stream));
+    note_launches(b->n);
     return QCB_OK;
 }
 

@@ -203,14 +203,27 @@ struct FmtImpl {
         return cudaGetLastError();
     }
     static cudaError_t aos_to_soa(const Geom& g, const double2* aos, void* links, int bswap, cudaStream_t s) {
-        const unsigned nb = (unsigned)((g.V * 4 + 255) / 256);
-        k_aos_to_soa<R, NE><<<nb, 256, 0, s>>>(g, aos, view(links, g.Vh), bswap);
+        k_aos_to_soa<R, NE><<<(unsigned)g.nT, kAosThreads, 0, s>>>(g, aos, view(links, g.Vh), bswap);
         return cudaGetLastError();
     }
     static cudaError_t soa_to_aos(const Geom& g, const void* links, double2* aos, int bswap, cudaStream_t s) {
-        const unsigned nb = (unsigned)((g.V * 4 + 255) / 256);
-        k_soa_to_aos<R, NE><<<nb, 256, 0, s>>>(g, view(links, g.Vh), aos, bswap);
+        k_soa_to_aos<R, NE><<<(unsigned)g.nT, kAosThreads, 0, s>>>(g, view(links, g.Vh), aos, bswap);
         return cudaGetLastError();
+    }
+    template <typename RS, int NES>
+    static cudaError_t convert_from(const Geom& g, const void* src, void* dst, cudaStream_t s) {
+        const dim3 grid((unsigned)((g.Vh + 255) / 256), 8);
+        k_convert<RS, NES, R, NE><<<grid, 256, 0, s>>>(g.Vh, FmtImpl<RS, NES>::view(src, g.Vh), view(dst, g.Vh));
+        return cudaGetLastError();
+    }
+    // this format's field from one of format `fmt`
+    static cudaError_t convert_links(const Geom& g, int fmt, const void* src, void* dst, cudaStream_t s) {
+        switch (fmt) {
+            case 0: return convert_from<double, 9>(g, src, dst, s);
+            case 1: return convert_from<double, 6>(g, src, dst, s);
+            case 2: return convert_from<float, 9>(g, src, dst, s);
+            default: return convert_from<float, 6>(g, src, dst, s);
+        }
     }
     static cudaError_t start(const Geom& g, void* links, int hot, uint64_t seed, cudaStream_t s) {
         k_start<R, NE><<<dim3((unsigned)((g.Vh + 127) / 128), 8), 128, 0, s>>>(g, view(links, g.Vh), hot, seed);
@@ -259,6 +272,7 @@ struct FmtImpl {
         o.unitarity = &unitarity;
         o.aos_to_soa = &aos_to_soa;
         o.soa_to_aos = &soa_to_aos;
+        o.convert_links = &convert_links;
         o.start = &start;
         o.shift = &shift;
         o.reunitarize = &reunitarize;
