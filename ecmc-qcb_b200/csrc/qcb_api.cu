@@ -240,16 +240,11 @@ int flow_step_meas(qcb_flow_s* fl) {
     return QCB_OK;
 }
 
-// The measurement of the flowed field alone through the measuring stage 1 (its stage-1 output, in
-// the spare buffer, is left unused): the last measurement of a run, so that every row of a measured
-// flow comes from the same arithmetic.
+// The measurement of the flowed field alone from the same clover halves: the last measurement of a run,
+// so that every row of a measured flow comes from the same arithmetic.
 int meas_halves_only(qcb_flow_s* fl) {
     qcb_field_s* f = fl->fld;
-    RET(ensure_alt(f));
-    const int rep = needs_reproject(f->prec, f->store);
-    RET(launch(f, QCB_K_CLOVER, [&] {
-        return fmt_ops(f->fmt).flow1_meas(f->g, f->links, f->alt, fl->z, fl->eps, rep, fl->halves, f->stream);
-    }));
+    RET(launch(f, QCB_K_CLOVER, [&] { return fmt_ops(f->fmt).meas_only(f->g, f->links, fl->halves, f->stream); }));
     const unsigned nb = halves_blocks(f->g.Vh);
     RET(launch(f, QCB_K_CLOVER,
                [&] { return fmt_ops(f->fmt).clover_halves(f->g, fl->halves, f->partials, nb, f->stream); }));
@@ -339,8 +334,8 @@ int flow_graph_run(qcb_flow_s* fl, int kind, int n_rk) {
 
 // One measurement of the flowed field -- q, e and the plaquette sum into the next row of the
 // measurement buffer -- followed by n_rk RK3 steps.  With the halves buffer in
-// place (measured flows with RK3 steps) the measurement comes from the measuring stage 1: that of
-// the following step, or for the last measurement one whose output is left unused.
+// place (measured flows with RK3 steps) the measurement comes from the measuring stage 1 of the
+// following step, or for the last one from the halves alone.
 int meas_block(qcb_flow_s* fl, int n_rk) {
     qcb_field_s* f = fl->fld;
     const bool fused = n_rk > 0 && fl->halves;

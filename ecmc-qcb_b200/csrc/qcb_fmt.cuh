@@ -130,6 +130,11 @@ struct FmtImpl {
         return launch_early(k_flow_stage1_meas<R, NE>, nb, QCB_FLOW_THREADS, s, g, view(win, g.Vh), view(wout, g.Vh), za,
                             eps, rep, H);
     }
+    static cudaError_t meas_only(const Geom& g, const void* w, void* hbuf, cudaStream_t s) {
+        const unsigned nb = 8u * (unsigned)((g.Vh + QCB_FLOW_THREADS - 1) / QCB_FLOW_THREADS);
+        return launch_early(k_meas_only<R, NE>, nb, QCB_FLOW_THREADS, s, g, view(w, g.Vh),
+                            HalfClovers<R>{(R*)hbuf, 2 * g.Vh});
+    }
     static cudaError_t clover_halves(const Geom& g, const void* hbuf, double* partials, unsigned nb, cudaStream_t s) {
         const HalfClovers<R> H{(R*)hbuf, 2 * g.Vh};
         return launch_early(k_clover_halves<R>, nb, 128, s, g, H, partials);
@@ -260,6 +265,7 @@ struct FmtImpl {
         o.probe_link = &probe_link;
         o.flow1 = &flow1;
         o.flow1_meas = &flow1_meas;
+        o.meas_only = &meas_only;
         o.flow_tiles1_meas = &flow_tiles1_meas;
         o.halves_tiles = &halves_tiles;
         o.clover_halves = &clover_halves;

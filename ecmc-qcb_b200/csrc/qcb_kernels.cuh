@@ -258,7 +258,8 @@ __device__ __forceinline__ void acc_product(const M3<R>& A, const M3<R>& B, R ou
 
 // staple_rt_rows, and for the planes this direction handles the two clover halves and the plaquette
 // trace of the link's site (see above).  u is the link U_mu(x) itself.
-template <typename R, int NE, bool EARLY>
+// ONLY: the halves and nothing else -- the planes of other directions are skipped, and A is not formed.
+template <typename R, int NE, bool EARLY, bool ONLY = false>
 __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkField<R, NE>& U, const int c[4],
                                                      int lex, int par, int mu, const M3<R>& u_in,
                                                      const HalfClovers<R>& H) {
@@ -273,6 +274,7 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
         const int nu = sizeof(R) == 8 ? mu ^ (k + 1) : (k < mu ? k : k + 1);
         const int plane = mu < nu ? plane_index(mu, nu) : plane_index(nu, mu);
         const bool owned = plane_owner(plane) == mu;
+        if (ONLY && !owned) continue;
         const int dnu = sel4(st.dn, nu);
         const int xnu = lex + sel4(st.up, nu);
         const int xmnu = lex + dnu;
@@ -299,13 +301,13 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
 #pragma unroll
                     for (int q = 0; q < 3; q++) cmac_nc(v, t[i][q], d(j, q));
                     Sf(i, j) = v;
-                    A(i, j) = A(i, j) + v;
+                    if (!ONLY) A(i, j) = A(i, j) + v;
                 }
 #pragma unroll
             for (int j = 0; j < 3; j++) {
                 const int j1 = (j + 1) % 3, j2 = (j + 2) % 3;
                 Sf(2, j) = conj_cross(Sf(0, j1), Sf(1, j2), Sf(0, j2), Sf(1, j1));
-                A(2, j) = A(2, j) + Sf(2, j);
+                if (!ONLY) A(2, j) = A(2, j) + Sf(2, j);
             }
         }
         M3<R> Sb;
@@ -330,13 +332,13 @@ __device__ __forceinline__ M3<R> staple_rt_rows_meas(const Geom& g, const LinkFi
 #pragma unroll
                     for (int q = 0; q < 3; q++) cmac_cn(v, t[q][i], v2(q, j));
                     Sb(i, j) = v;
-                    A(i, j) = A(i, j) + v;
+                    if (!ONLY) A(i, j) = A(i, j) + v;
                 }
 #pragma unroll
             for (int j = 0; j < 3; j++) {
                 const int j1 = (j + 1) % 3, j2 = (j + 2) % 3;
                 Sb(2, j) = conj_cross(Sb(0, j1), Sb(1, j2), Sb(0, j2), Sb(1, j1));
-                A(2, j) = A(2, j) + Sb(2, j);
+                if (!ONLY) A(2, j) = A(2, j) + Sb(2, j);
             }
         }
         if (owned) {
@@ -1096,6 +1098,25 @@ __global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MEAS_MINB(R))
     flow_map<R>(blockIdx.x, mu, par, h);
     if (h >= g.Vh) return;
     flow_link<R, NE, 1, true, true>(g, Win, Wout, Z, eps, mu, par, (int)h, reproject, H);
+}
+
+// The clover halves of a configuration alone, as k_flow_stage1_meas writes them (the same operations, bit
+// for bit): the last measurement of a flow, which no step follows.  Half of the staples (each plane once)
+// and no exponential, no links and no accumulator written: about 0.39 ms less than the measuring stage at 32^4
+// in FP64 and 0.33-0.7 ms in FP32 (six measurements with five steps 12.7 to 12.3 ms, 7.6 to 6.9 ms).
+template <typename R, int NE>
+__global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MEAS_MINB(R))
+    k_meas_only(Geom g, LinkField<R, NE> W, HalfClovers<R> H) {
+    int mu, par;
+    int64_t h;
+    flow_map<R>(blockIdx.x, mu, par, h);
+    if (h >= g.Vh) return;
+    int c[4];
+    site_coords(g, par, (uint32_t)h, c);
+    cudaGridDependencySynchronize();
+    M3<R> u;
+    if (sizeof(R) == 4) u = W.load(mu, par, (int)h);
+    staple_rt_rows_meas<R, NE, true, true>(g, W, c, lex_of(g, c), par, mu, u, H);
 }
 
 // ------------------------------------------------------------------ the reference's separate flow passes

@@ -37,8 +37,8 @@
 #include "qcb_ops.h"
 
 // Requests take every measurement from a measuring stage 1 (clover halves), as qcb_flow_measure
-// does: that of the RK3 step that follows it, or for the last one a stage 1 whose output is left
-// unused; 0 measures with clover passes.
+// does: that of the RK3 step that follows it, or for the last one the halves alone (a small request's
+// last one rides in the shared stage 1, its flow output left unused); 0 measures with clover passes.
 #ifndef QCB_SERVE_FUSED_MEAS
 #define QCB_SERVE_FUSED_MEAS 1
 #endif
@@ -299,7 +299,7 @@ bool measure_big(qcb_server_s* s, Request* r, int flip_xor) {
 // Stage 1 of a big request's RK3 step that also measures its input, into r->meas_slot: the
 // measuring stage 1, the per-site sum of the clover halves and the finalize of qcb_flow_measure
 // (same kernels, same partial counts), so a big request's rows equal the plain measured flow's.
-bool flow_big_meas(qcb_server_s* s, Request* r, int flip_xor, int rep) {
+bool flow_big_meas(qcb_server_s* s, Request* r, int flip_xor, int rep, bool last = false) {
     const int f = (r->flip ^ flip_xor) & 1;
     void* a = r->buf;
     void* b = (char*)r->buf + r->off_out;
@@ -307,8 +307,9 @@ bool flow_big_meas(qcb_server_s* s, Request* r, int flip_xor, int rep) {
     if (!grow(s, &s->halves, &s->halves_cap, halves_bytes(s->fmt, r->g.Vh))) return false;
     if (!grow(s, &s->big_partials, &s->big_partials_cap, (size_t)nb * 3)) return false;
     const FmtOps& o = fmt_ops(s->fmt);
-    if (!cuda_ok(s, o.flow1_meas(r->g, (f & 1) ? b : a, (f & 1) ? a : b, (char*)r->buf + r->off_z, r->eps, rep,
-                                 s->halves, s->stream),
+    void* win = f ? b : a;
+    if (!cuda_ok(s, last ? o.meas_only(r->g, win, s->halves, s->stream)
+                         : o.flow1_meas(r->g, win, f ? a : b, (char*)r->buf + r->off_z, r->eps, rep, s->halves, s->stream),
                  "flow launch"))
         return false;
     if (!cuda_ok(s, o.clover_halves(r->g, s->halves, s->big_partials, nb, s->stream), "clover launch")) return false;
@@ -454,11 +455,11 @@ bool big_tick(qcb_server_s* s, int rep) {
     const int fx = (int)(s->nflow_b & 1);
     bool ok = true;
     // a big request that flows on after this measurement takes it from its next stage 1; its last
-    // measurement runs a measuring stage 1 now, whose output is left unused
+    // measurement is taken now, from the halves alone
     for (Request* r : s->big) {
         if (QCB_SERVE_FUSED_MEAS) {
             r->meas_slot = (double*)((char*)r->buf + r->off_meas) + (size_t)(s->tick_b - r->tick0) * 3;
-            if (s->tick_b - r->tick0 == r->n_steps - 1) ok = ok && flow_big_meas(s, r, fx, rep);
+            if (s->tick_b - r->tick0 == r->n_steps - 1) ok = ok && flow_big_meas(s, r, fx, rep, true);
         } else {
             ok = ok && measure_big(s, r, fx);
         }

@@ -151,8 +151,8 @@ int qcb_flow_rk3(qcb_flow fl, int n);
  * times { measure (Q, E) ; if not last: n_rk RK3 steps }; tQE receives 3*n_steps doubles
  * (t, Q, E).  If plaq is non-NULL it receives n_steps plaquettes measured beside Q, E.  With
  * n_rk > 0 every measurement is taken from a measuring RK3 stage 1 (the clover from the force's
- * staple differences): that of the step that follows it, for the last one a stage 1 whose output
- * is left unused; with n_rk = 0, from a clover pass.  The first call with n_rk > 0 allocates the
+ * staple differences): that of the step that follows it, for the last one the same staple
+ * differences alone; with n_rk = 0, from a clover pass.  The first call with n_rk > 0 allocates the
  * flow state's buffer for it (114 reals a site in the flow's precision). */
 int qcb_flow_measure(qcb_flow fl, qcb_field src, int n_steps, int n_rk, double* tQE, double* plaq);
 /* The flowed field (GradientFlow::field_c); owned by the flow state. */
