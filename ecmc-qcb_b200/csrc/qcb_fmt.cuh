@@ -195,8 +195,16 @@ struct FmtImpl {
         return cudaGetLastError();
     }
 
-    static cudaError_t plaquette(const Geom& g, const void* links, double* partials, unsigned nbx, cudaStream_t s) {
-        k_plaquette<R, NE><<<dim3(2, nbx), 256, 0, s>>>(g, view(links, g.Vh), partials);
+    // blocks of the plaquette sum (one partial each)
+    static unsigned plaquette_blocks(const Geom& g) {
+        if (sizeof(R) == 8) return (unsigned)std::min(2 * g.nT, 16 * 148);
+        return 2u * (unsigned)std::min<int64_t>((g.Vh + 255) / 256, 148 * 8);
+    }
+    static cudaError_t plaquette(const Geom& g, const void* links, double* partials, cudaStream_t s) {
+        const unsigned nb = plaquette_blocks(g);
+        if constexpr (sizeof(R) == 8)
+            return launch_early(k_plaquette_planes<NE>, nb, kPlaqThreads, s, g, view(links, g.Vh), partials);
+        k_plaquette<R, NE><<<dim3(2, nb / 2), 256, 0, s>>>(g, view(links, g.Vh), partials);
         return cudaGetLastError();
     }
     static cudaError_t clover(const Geom& g, const void* links, double* partials, unsigned nbx, cudaStream_t s) {
@@ -274,6 +282,7 @@ struct FmtImpl {
         o.flow_replace = &flow_replace;
         o.clover_site = &clover_site;
         o.plaquette = &plaquette;
+        o.plaquette_blocks = &plaquette_blocks;
         o.clover = &clover;
         o.unitarity = &unitarity;
         o.aos_to_soa = &aos_to_soa;

@@ -65,6 +65,10 @@ struct TimedLaunch {
 // 12-real heatbath chain diverged after ~180 sweeps).
 inline int needs_reproject(int prec, int store) { return (prec == QCB_PREC_F32 || store == QCB_STORE_12) ? 1 : 0; }
 
+namespace qcb {
+constexpr int kResDoubles = 64;
+}
+
 struct qcb_field_s {
     int L[4];
     qcb::Geom g;
@@ -82,9 +86,9 @@ struct qcb_field_s {
     bool own_stream = false;
     double* partials = nullptr;
     size_t partials_cap = 0;  // doubles
-    double* d_res = nullptr;  // device results (8 doubles)
-    double* h_res = nullptr;  // pinned host results (8 doubles)
-    int* d_err = nullptr;     // device error flags
+    double* d_res = nullptr;  // device results (kResDoubles, the last one the error flags)
+    double* h_res = nullptr;  // pinned host copy of them
+    int* d_err = nullptr;     // device error flags (in d_res)
     bool timing = false;
     std::vector<qcb::TimedLaunch> pending;
     std::vector<cudaEvent_t> event_pool;

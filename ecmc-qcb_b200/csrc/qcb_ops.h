@@ -71,7 +71,8 @@ struct FmtOps {
     cudaError_t (*flow_replace)(const Geom& g, void* f0, const void* f1, cudaStream_t s);
     cudaError_t (*clover_site)(const Geom& g, const void* links, int par, int h, int mu, int nu, double* out,
                                cudaStream_t s);
-    cudaError_t (*plaquette)(const Geom& g, const void* links, double* partials, unsigned nbx, cudaStream_t s);
+    unsigned (*plaquette_blocks)(const Geom& g);  // partials of `plaquette`
+    cudaError_t (*plaquette)(const Geom& g, const void* links, double* partials, cudaStream_t s);
     cudaError_t (*clover)(const Geom& g, const void* links, double* partials, unsigned nbx, cudaStream_t s);
     cudaError_t (*unitarity)(const Geom& g, const void* links, double* partials, unsigned nbx, cudaStream_t s);
     cudaError_t (*aos_to_soa)(const Geom& g, const double2* aos, void* links, int bswap, cudaStream_t s);
