@@ -223,6 +223,10 @@ struct FmtImpl {
         k_soa_to_aos<R, NE><<<(unsigned)g.nT, kAosThreads, 0, s>>>(g, view(links, g.Vh), aos, bswap);
         return cudaGetLastError();
     }
+    static cudaError_t packed_to_soa(const Geom& g, const void* aos, void* links, cudaStream_t s) {
+        k_packed_to_soa<R, NE><<<(unsigned)g.nT, kAosThreads, 0, s>>>(g, (const typename V2<R>::T*)aos, view(links, g.Vh));
+        return cudaGetLastError();
+    }
     template <typename RS, int NES>
     static cudaError_t convert_from(const Geom& g, const void* src, void* dst, cudaStream_t s) {
         const dim3 grid((unsigned)((g.Vh + 255) / 256), 8);
@@ -288,6 +292,7 @@ struct FmtImpl {
         o.aos_to_soa = &aos_to_soa;
         o.soa_to_aos = &soa_to_aos;
         o.convert_links = &convert_links;
+        o.packed_to_soa = &packed_to_soa;
         o.start = &start;
         o.shift = &shift;
         o.reunitarize = &reunitarize;

@@ -1663,6 +1663,41 @@ __global__ void __launch_bounds__(kAosThreads) k_soa_to_aos(Geom g, LinkField<R,
     }
 }
 
+// Links in AoS order that hold this format's reals only (NE complexes of R a link: the requests' host
+// buffers) into the tiles, as k_aos_to_soa moves full FP64 links.
+template <typename R, int NE>
+__global__ void __launch_bounds__(kAosThreads) k_packed_to_soa(Geom g, const typename V2<R>::T* __restrict__ aos,
+                                                               LinkField<R, NE> U) {
+    typedef typename V2<R>::T C2;
+    constexpr int kPair = 8 * NE + 1;
+    __shared__ C2 sm[32 * kPair];
+    const int64_t first = (int64_t)blockIdx.x * 32, left = g.Vh - first;
+    const int n = 8 * NE * (int)(left < 32 ? left : 32);
+    const C2* run = aos + first * (8 * NE);
+    constexpr int N = 32 * 8 * NE / kAosThreads;
+    C2 v[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const int i = threadIdx.x + k * kAosThreads;
+        if (i < n) v[k] = __ldcs(run + i);
+    }
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const int i = threadIdx.x + k * kAosThreads;
+        if (i < n) sm[i + i / (8 * NE)] = v[k];
+    }
+    __syncthreads();
+    const int w = threadIdx.x >> 5, mu = w >> 1, par = w & 1, h = (int)first + (threadIdx.x & 31);
+    if (h >= g.Vh) return;
+    int c[4];
+    site_coords(g, par, (uint32_t)h, c);
+    const C2* p = sm + (h & 31) * kPair + (c[0] & 1) * 4 * NE + mu * NE;
+    M3<R> u;
+#pragma unroll
+    for (int e = 0; e < NE; e++) u.e[e] = mkc<R>(p[e].x, p[e].y);
+    U.store(mu, par, h, u);
+}
+
 // A field in another storage format: every entry through double, as an export and an import would.
 // One pass over both fields (32^4 FP64-18 to FP32-18 136 us) where an export to and an import from a staging
 // buffer of AoS links took 431 us.

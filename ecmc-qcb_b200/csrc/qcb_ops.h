@@ -77,6 +77,8 @@ struct FmtOps {
     cudaError_t (*unitarity)(const Geom& g, const void* links, double* partials, unsigned nbx, cudaStream_t s);
     cudaError_t (*aos_to_soa)(const Geom& g, const double2* aos, void* links, int bswap, cudaStream_t s);
     cudaError_t (*soa_to_aos)(const Geom& g, const void* links, double2* aos, int bswap, cudaStream_t s);
+    // AoS links holding the format's reals only (link_reals of qcb_serve.cu's host buffers)
+    cudaError_t (*packed_to_soa)(const Geom& g, const void* aos, void* links, cudaStream_t s);
     // links of this format from a field of storage format src_fmt of the same lattice
     cudaError_t (*convert_links)(const Geom& g, int src_fmt, const void* src, void* dst, cudaStream_t s);
     cudaError_t (*start)(const Geom& g, void* links, int hot, uint64_t seed, cudaStream_t s);
