@@ -1,7 +1,7 @@
 // qcb_batch.cu -- many independent heatbath chains advanced together.
 //
 // A batch holds n lattices of (possibly) different sizes and couplings in one device arena.
-// Each (parity, mu) phase of a sweep is ONE persistent launch over the tile work list of all
+// Each (parity, mu) phase of a sweep is ONE launch over the tile work list of all
 // chains (k_hb_tiles); a whole sweep -- 8 phases plus the device-side sweep counter increment --
 // is captured once as a CUDA graph and replayed.  Chain i draws from the Philox link streams
 // keyed on its own seed, with the batch's sweep counter, so it receives exactly the numbers a

@@ -31,11 +31,9 @@ struct FmtImpl {
     template <int MU, int BLOCK, int MINB>
     static cudaError_t hb_launch(const WorkList& w, int par, int n_hits, const uint32_t* sweep_dev, uint32_t sweep_add,
                                  int reproject, int* err, cudaStream_t s) {
-        static int cache = 0;
         auto k = k_hb_tiles<R, NE, MU, BLOCK, MINB>;
-        const int64_t need = ((int64_t)w.nb_total * TILE + BLOCK - 1) / BLOCK;
-        const int grid = (int)std::min<int64_t>(need, resident_blocks(k, BLOCK, &cache));
-        k<<<grid, BLOCK, 0, s>>>(w.lats, w.tile_lat, w.one, w.nb_total, par, n_hits, sweep_dev, sweep_add, reproject, err);
+        const int64_t grid = ((int64_t)w.nb_total * TILE + BLOCK - 1) / BLOCK;
+        k<<<(unsigned)grid, BLOCK, 0, s>>>(w.lats, w.tile_lat, w.one, w.nb_total, par, n_hits, sweep_dev, sweep_add, reproject, err);
         return cudaGetLastError();
     }
     template <int MU>

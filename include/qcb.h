@@ -249,7 +249,7 @@ void* qcb_batch_stream(qcb_batch b);
 /* hot_start / cold_start of every chain (chain i as qcb_hot_start(field, seed[i])). */
 int qcb_batch_hot_start(qcb_batch b);
 int qcb_batch_cold_start(qcb_batch b);
-/* n_sweeps full sweeps of every chain.  Each (parity, mu) phase of all chains is one persistent
+/* n_sweeps full sweeps of every chain.  Each (parity, mu) phase of all chains is one
  * launch over a tile work list; one sweep (8 phases + the device sweep counter) is captured as a
  * CUDA graph at the first call with a given n_hits / launch shape and replayed. */
 int qcb_batch_sweep(qcb_batch b, int n_hits, int n_sweeps);
