@@ -15,19 +15,6 @@ struct FmtImpl {
         return f;
     }
 
-    // Resident-grid size of a persistent kernel: blocks per SM (occupancy) x SMs, cached per
-    // kernel instance.
-    template <typename K>
-    static int resident_blocks(K kernel, int block, int* cache) {
-        if (*cache == 0) {
-            int per_sm = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0) != cudaSuccess || per_sm < 1)
-                per_sm = 1;
-            *cache = per_sm * sm_count();
-        }
-        return *cache;
-    }
-
     template <int MU, int BLOCK, int MINB>
     static cudaError_t hb_launch(const WorkList& w, int par, int n_hits, const uint32_t* sweep_dev, uint32_t sweep_add,
                                  int reproject, int* err, cudaStream_t s) {
@@ -58,11 +45,9 @@ struct FmtImpl {
 
     template <int STAGE>
     static cudaError_t flow_launch(const WorkList& w, int flip_xor, int rep, cudaStream_t s) {
-        static int cache = 0;
         auto k = k_flow_tiles<R, NE, STAGE>;
         const int ntiles = 8 * w.nb_total;
-        const int grid = std::min(ntiles, resident_blocks(k, QCB_FLOW_THREADS, &cache));
-        k<<<grid, QCB_FLOW_THREADS, 0, s>>>(w.lats, w.tile_lat, w.one, ntiles, flip_xor, rep);
+        k<<<ntiles, QCB_FLOW_THREADS, 0, s>>>(w.lats, w.tile_lat, w.one, flip_xor, rep);
         return cudaGetLastError();
     }
     static cudaError_t flow(const WorkList& w, int stage, int flip_xor, int rep, cudaStream_t s) {
@@ -167,7 +152,7 @@ struct FmtImpl {
         return cudaGetLastError();
     }
 
-    // Reduction work lists are not persistent: one block per tile, one partial per tile.
+    // Reductions: one partial per tile.
     static cudaError_t plaq_tiles(const WorkList& w, int flip_xor, double* partials, cudaStream_t s) {
         const int ntiles = 2 * w.nb_total;
         k_plaq_tiles<R, NE><<<ntiles, TILE, 0, s>>>(w.lats, w.tile_lat, w.one, ntiles, flip_xor, partials);
@@ -180,11 +165,9 @@ struct FmtImpl {
     }
 
     static cudaError_t flow_tiles1_meas(const WorkList& w, int flip_xor, int rep, cudaStream_t s) {
-        static int cache = 0;
         auto k = k_flow_tiles1_meas<R, NE>;
         const int ntiles = 8 * w.nb_total;
-        const int grid = std::min(ntiles, resident_blocks(k, QCB_FLOW_THREADS, &cache));
-        k<<<grid, QCB_FLOW_THREADS, 0, s>>>(w.lats, w.tile_lat, w.one, ntiles, flip_xor, rep);
+        k<<<ntiles, QCB_FLOW_THREADS, 0, s>>>(w.lats, w.tile_lat, w.one, flip_xor, rep);
         return cudaGetLastError();
     }
     static cudaError_t halves_tiles(const WorkList& w, double* partials, cudaStream_t s) {

@@ -7,7 +7,7 @@
 //     the server's own stream-ordered pool and returns to it when a request completes;
 //   * one scheduler tick measures Q/E of every resident request and then advances every
 //     resident request by n_rk RK3 steps.  Requests below kBigVh half-sites share one batched
-//     clover launch (with a per-request finalize) and three persistent launches per RK3 step over
+//     clover launch (with a per-request finalize) and three launches per RK3 step over
 //     the tile work list of all of them, so requests that arrive while others are on the GPU
 //     share the same launches; a request of kBigVh half-sites or more fills the GPU by itself and
 //     runs the single-lattice kernels (geometry in kernel parameters, no per-tile descriptor

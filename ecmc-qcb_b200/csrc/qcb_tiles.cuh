@@ -4,8 +4,9 @@
 // single field).  Lattice i owns nb_i = ceil(V_i / 2 / TILE) "blocks" of half-sites; a kernel
 // of kind m (m = 1 heatbath, 8 flow, 2 plaquette, 6 clover) sees m * nb_i tiles for that lattice,
 // stored contiguously from tile m * nb_begin_i.  tile_lat maps a block index (t / m) to its
-// lattice; with a single lattice it is NULL.  Kernels are persistent: a grid sized to the
-// resident capacity of the GPU walks the list with a stride of gridDim.x.
+// lattice; with a single lattice it is NULL.  One block per tile: a resident grid that walked the
+// list in strides was slower for the heatbath (below) and the flow (24 requests of 16^4 with 100
+// measured steps 262 against 254 ms FP32-18, 253 against 235 FP32-12).
 #pragma once
 #include "qcb_kernels.cuh"
 
@@ -73,23 +74,22 @@ __global__ void __launch_bounds__(BLOCK, MINB)
 // when (f + s - 1) is even; a whole RK3 step therefore moves the field to the other buffer.
 template <typename R, int NE, int STAGE>
 __global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MINB(R))
-    k_flow_tiles(const LatDesc* __restrict__ lats, const int* __restrict__ tile_lat, const LatDesc one, int ntiles,
-                 int flip_xor, int reproject) {
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const LatDesc* d = lattice_of(lats, tile_lat, one, t >> 3);
-        const Geom g = d->g;
-        int mu, par;
-        int64_t h;
-        flow_map<R>(t - 8 * d->nb_begin, mu, par, h);
-        if (h >= g.Vh) continue;
-        const bool in_b = (((d->flip ^ flip_xor) + STAGE - 1) & 1) != 0;
-        const LinkField<R, NE> win = lview<R, NE>(in_b ? d->links_out : d->links, g.Vh);
-        const LinkField<R, NE> wout = lview<R, NE>(in_b ? d->links : d->links_out, g.Vh);
-        AlgField<R> z;
-        z.p = (typename AlgField<R>::C2*)d->z;
-        z.Vh = g.Vh;
-        flow_link<R, NE, STAGE>(g, win, wout, z, d->eps, mu, par, (int)h, reproject);
-    }
+    k_flow_tiles(const LatDesc* __restrict__ lats, const int* __restrict__ tile_lat, const LatDesc one, int flip_xor,
+                 int reproject) {
+    const int t = blockIdx.x;
+    const LatDesc* d = lattice_of(lats, tile_lat, one, t >> 3);
+    const Geom g = d->g;
+    int mu, par;
+    int64_t h;
+    flow_map<R>(t - 8 * d->nb_begin, mu, par, h);
+    if (h >= g.Vh) return;
+    const bool in_b = (((d->flip ^ flip_xor) + STAGE - 1) & 1) != 0;
+    const LinkField<R, NE> win = lview<R, NE>(in_b ? d->links_out : d->links, g.Vh);
+    const LinkField<R, NE> wout = lview<R, NE>(in_b ? d->links : d->links_out, g.Vh);
+    AlgField<R> z;
+    z.p = (typename AlgField<R>::C2*)d->z;
+    z.Vh = g.Vh;
+    flow_link<R, NE, STAGE>(g, win, wout, z, d->eps, mu, par, (int)h, reproject);
 }
 
 // Stage 1 that also writes each lattice's clover halves (the serving tick's measurement; see
@@ -97,23 +97,22 @@ __global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MINB(R))
 template <typename R, int NE>
 __global__ void __launch_bounds__(QCB_FLOW_THREADS, QCB_FLOW_MEAS_MINB(R))
     k_flow_tiles1_meas(const LatDesc* __restrict__ lats, const int* __restrict__ tile_lat, const LatDesc one,
-                       int ntiles, int flip_xor, int reproject) {
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const LatDesc* d = lattice_of(lats, tile_lat, one, t >> 3);
-        const Geom g = d->g;
-        int mu, par;
-        int64_t h;
-        flow_map<R>(t - 8 * d->nb_begin, mu, par, h);
-        if (h >= g.Vh) continue;
-        const bool in_b = ((d->flip ^ flip_xor) & 1) != 0;
-        const LinkField<R, NE> win = lview<R, NE>(in_b ? d->links_out : d->links, g.Vh);
-        const LinkField<R, NE> wout = lview<R, NE>(in_b ? d->links : d->links_out, g.Vh);
-        AlgField<R> z;
-        z.p = (typename AlgField<R>::C2*)d->z;
-        z.Vh = g.Vh;
-        const HalfClovers<R> H{(R*)d->halves, 2 * g.Vh};
-        flow_link<R, NE, 1, true>(g, win, wout, z, d->eps, mu, par, (int)h, reproject, H);
-    }
+                       int flip_xor, int reproject) {
+    const int t = blockIdx.x;
+    const LatDesc* d = lattice_of(lats, tile_lat, one, t >> 3);
+    const Geom g = d->g;
+    int mu, par;
+    int64_t h;
+    flow_map<R>(t - 8 * d->nb_begin, mu, par, h);
+    if (h >= g.Vh) return;
+    const bool in_b = ((d->flip ^ flip_xor) & 1) != 0;
+    const LinkField<R, NE> win = lview<R, NE>(in_b ? d->links_out : d->links, g.Vh);
+    const LinkField<R, NE> wout = lview<R, NE>(in_b ? d->links : d->links_out, g.Vh);
+    AlgField<R> z;
+    z.p = (typename AlgField<R>::C2*)d->z;
+    z.Vh = g.Vh;
+    const HalfClovers<R> H{(R*)d->halves, 2 * g.Vh};
+    flow_link<R, NE, 1, true>(g, win, wout, z, d->eps, mu, par, (int)h, reproject, H);
 }
 
 // ---------------------------------------------------------------- per-tile reductions

@@ -271,7 +271,7 @@ int qcb_batch_tune(qcb_batch b, int n_hits, int n_trial, int allow_store_change,
 /* Continuous-batching service for topo_charge_flowed (src/observables/observables_mpi.cpp:159-186):
  * requests of any lattice size are queued, admitted in order as the HBM budget allows, and every
  * scheduler tick measures (Q, E) of all resident requests and advances them by n_rk RK3 steps in
- * shared persistent launches.  Runs its own scheduler thread on the current device.
+ * shared launches.  Runs its own scheduler thread on the current device.
  * max_active <= 0: no limit besides the budget.  Every request takes its measurements from
  * measuring RK3 stage 1 launches, as qcb_flow_measure does; a request below 2^17 half-sites holds
  * 114 reals a site for them within its memory, and for the larger ones, which run alone, the server
