@@ -285,6 +285,19 @@ QCB_HD void ch_coeffs(double t, double d, double q[6]) {
         ch_horner<18>(t, d, q);
 }
 
+// The invariants t and d of the exponential below, in double.
+template <typename R>
+QCB_HD void su3_invariants(const AntiH<R>& X, double& t, double& d) {
+    const double x01r = X.o[0].re, x01i = X.o[0].im, x02r = X.o[1].re, x02i = X.o[1].im;
+    const double x12r = X.o[2].re, x12i = X.o[2].im;
+    const double a0 = X.d[0], a1 = X.d[1], a2 = X.d[2];
+    const double n01 = fma(x01r, x01r, x01i * x01i), n02 = fma(x02r, x02r, x02i * x02i);
+    const double n12 = fma(x12r, x12r, x12i * x12i);
+    t = (n01 + n02) + n12 + 0.5 * (fma(a0, a0, fma(a1, a1, a2 * a2)));
+    const double pr = fma(x01r, x12r, -x01i * x12i), pi = fma(x01r, x12i, x01i * x12r);  // X01 X12
+    const double im3 = fma(pi, x02r, -pr * x02i);                                         // Im(p conj(X02))
+    d = fma(a0 * a1, a2, fma(2.0, im3, -fma(a0, n12, fma(a1, n02, a2 * n01))));
+}
 // exp_su3_luscher (src/su3/utils.cpp:145-193): exp(X) of a traceless anti-Hermitian X by the
 // Cayley-Hamilton form q0 + q1 X + q2 X^2 with the Horner recurrence above.  The invariants
 //   t = |X01|^2 + |X02|^2 + |X12|^2 + (a0^2 + a1^2 + a2^2)/2,
@@ -299,17 +312,7 @@ QCB_HD M3<R> exp_su3(const AntiH<R>& X) {
     const Cx<R>* o = X.o;
     const R* a = X.d;
     double t, d;
-    {
-        const double x01r = o[0].re, x01i = o[0].im, x02r = o[1].re, x02i = o[1].im;
-        const double x12r = o[2].re, x12i = o[2].im;
-        const double a0 = a[0], a1 = a[1], a2 = a[2];
-        const double n01 = fma(x01r, x01r, x01i * x01i), n02 = fma(x02r, x02r, x02i * x02i);
-        const double n12 = fma(x12r, x12r, x12i * x12i);
-        t = (n01 + n02) + n12 + 0.5 * (fma(a0, a0, fma(a1, a1, a2 * a2)));
-        const double pr = fma(x01r, x12r, -x01i * x12i), pi = fma(x01r, x12i, x01i * x12r);  // X01 X12
-        const double im3 = fma(pi, x02r, -pr * x02i);                                         // Im(p conj(X02))
-        d = fma(a0 * a1, a2, fma(2.0, im3, -fma(a0, n12, fma(a1, n02, a2 * n01))));
-    }
+    su3_invariants(X, t, d);
     double q[6];
     ch_coeffs<R>(t, d, q);
     const Cx<R> q0 = mkc<R>((R)q[0], (R)q[1]), q1 = mkc<R>((R)q[2], (R)q[3]), q2 = mkc<R>((R)q[4], (R)q[5]);
@@ -350,16 +353,80 @@ QCB_HD M3<R> exp_su3(const AntiH<R>& X) {
     return E;
 }
 
-// exp of a traceless anti-Hermitian matrix given as nine complexes.
+// 3x3 determinant by cofactor expansion along the first row.
 template <typename R>
-QCB_HD M3<R> exp_su3(const M3<R>& X) {
+QCB_HD Cx<R> det3(const M3<R>& m) {
+    Cx<R> c0 = m(1, 1) * m(2, 2) - m(1, 2) * m(2, 1);
+    Cx<R> c1 = m(1, 0) * m(2, 2) - m(1, 2) * m(2, 0);
+    Cx<R> c2 = m(1, 0) * m(2, 1) - m(1, 1) * m(2, 0);
+    return (m(0, 0) * c0 - m(0, 1) * c1) + m(0, 2) * c2;
+}
+
+// The nine reals of an anti-Hermitian matrix given as nine complexes.
+template <typename R>
+QCB_HD AntiH<R> upper_triangle(const M3<R>& X) {
     AntiH<R> a;
     a.o[0] = X(0, 1);
     a.o[1] = X(0, 2);
     a.o[2] = X(1, 2);
 #pragma unroll
     for (int i = 0; i < 3; i++) a.d[i] = X(i, i).im;
-    return exp_su3(a);
+    return a;
+}
+
+// exp_su3 of a matrix given as nine complexes (the diagnostic entry point): the nine reals where it is exactly
+// anti-Hermitian, else the same form with full products, which is what such a matrix has always got.
+template <typename R>
+QCB_HD M3<R> exp_su3_full(const M3<R>& X) {
+    // X^2 is Hermitian: compute the upper triangle and mirror it.
+    M3<R> X2;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = i; j < 3; j++) {
+            Cx<R> s = X(i, 0) * X(0, j);
+            cmac(s, X(i, 1), X(1, j));
+            cmac(s, X(i, 2), X(2, j));
+            X2(i, j) = s;
+        }
+    X2(1, 0) = cconj(X2(0, 1));
+    X2(2, 0) = cconj(X2(0, 2));
+    X2(2, 1) = cconj(X2(1, 2));
+    X2(0, 0).im = X2(1, 1).im = X2(2, 2).im = R(0);
+    double t, d;
+    if constexpr (sizeof(R) == sizeof(double)) {
+        const M3<double> Xd = convert<double>(X);
+        t = -0.5 * (((double)X2(0, 0).re + (double)X2(1, 1).re) + (double)X2(2, 2).re);
+        d = -det3(Xd).im;  // Re(i * det X)
+    } else {
+        su3_invariants(upper_triangle(X), t, d);
+    }
+    double q[6];
+    ch_horner<18>(t, d, q);
+    Cx<R> q0 = mkc<R>((R)q[0], (R)q[1]), q1 = mkc<R>((R)q[2], (R)q[3]), q2 = mkc<R>((R)q[4], (R)q[5]);
+    M3<R> E;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        Cx<R> v = q1 * X.e[k];
+        cmac(v, q2, X2.e[k]);
+        E.e[k] = v;
+    }
+    E(0, 0) = E(0, 0) + q0;
+    E(1, 1) = E(1, 1) + q0;
+    E(2, 2) = E(2, 2) + q0;
+    return E;
+}
+template <typename R>
+QCB_HD M3<R> exp_su3(const M3<R>& X) {
+    bool anti = true;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        anti = anti && X(i, i).re == R(0);
+#pragma unroll
+        for (int j = 0; j < i; j++) anti = anti && X(i, j).re == -X(j, i).re && X(i, j).im == X(j, i).im;
+    }
+    if (!anti) return exp_su3_full(X);
+    return exp_su3(upper_triangle(X));
 }
 
 // projection_su3 (src/gauge/GaugeField.cpp:36-58): column Gram-Schmidt, c2 = conj(c0 x c1).

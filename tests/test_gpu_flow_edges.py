@@ -3,6 +3,8 @@
 Lattices whose half-volume is below, at and just past multiples of the 32-site tiles and of the block
 shapes, every storage, against the oracle's RK3 steps.
 """
+import math
+
 import numpy as np
 import pytest
 
@@ -45,3 +47,21 @@ def test_exp_on_both_sides_of_the_series_rule(gpu, orc, prec, tol):
         X = Z * np.sqrt(want / t)[:, None, None]
         ref = np.stack([orc.exp_su3(x, 1.0) for x in X])
         assert np.max(np.abs(gpu.exp_su3(X, 1.0, prec) - ref)) < tol, want
+
+
+def test_exp_of_a_matrix_off_the_algebra(gpu, orc):
+    """The diagnostic exponential takes any matrix.  One with a part of 0.1 outside the algebra gets the
+    Cayley-Hamilton form of its own entries: X^2 from the upper triangle of the full product, t from its
+    trace, d from the full determinant.  Some forty FP64 operations on entries of order one: 1e-14."""
+    rng = np.random.default_rng(6)
+    noise = rng.normal(size=(2, 16, 3, 3))
+    X = np.stack([orc.proj_lie_su3(z) for z in noise[0] + 1j * noise[1]]) * 0.3
+    X = X + 0.1 * (rng.normal(size=X.shape) + 1j * rng.normal(size=X.shape))
+    up = np.triu(X @ X, 1)
+    X2 = up + np.conj(np.swapaxes(up, 1, 2)) + np.einsum("nii->ni", (X @ X).real)[:, :, None] * np.eye(3)
+    t, d = -0.5 * np.einsum("nii->n", X2).real, -np.linalg.det(X).imag
+    q0, q1, q2 = (np.zeros(16, complex) for _ in range(3))
+    for n in range(18, -1, -1):
+        q0, q1, q2 = 1 / math.factorial(n) - 1j * d * q2, q0 - t * q2, q1
+    ref = q0[:, None, None] * np.eye(3) + q1[:, None, None] * X + q2[:, None, None] * X2
+    assert np.max(np.abs(gpu.exp_su3(X, 1.0) - ref)) < 1e-14
