@@ -413,8 +413,8 @@ __device__ __forceinline__ AntiH<R> neg_proj_lie_mul(const M3<R>& u, const M3<R>
 #ifndef QCB_FLOW_MINB
 #define QCB_FLOW_MINB(R) (sizeof(R) == 8 ? 3 : 5)
 #endif
-// Clover kernels: 2 resident blocks per SM for FP64, 4 for FP32 (32^4 clover pass 1.02 ms FP64 and
-// 0.49 ms FP32 against 1.24 ms and 0.69 ms at 3 and 6).
+// Clover kernels: 2 resident blocks per SM for FP64, 4 for FP32 (32^4 clover pass 0.604 ms FP64 against 0.635
+// at 3; 0.49 ms FP32 against 0.69 ms at 6).
 #ifndef QCB_CLOVER_MINB
 #define QCB_CLOVER_MINB(R) (sizeof(R) == 8 ? 2 : 4)
 #endif
@@ -425,12 +425,6 @@ __device__ __forceinline__ AntiH<R> neg_proj_lie_mul(const M3<R>& u, const M3<R>
 // (FP64 3 blocks/SM with the link reloaded for the halves, no spills; FP32 4)
 #ifndef QCB_FLOW_MEAS_MINB
 #define QCB_FLOW_MEAS_MINB(R) (sizeof(R) == 8 ? 3 : 4)
-#endif
-// FP64 clover leaves with two-row products (third row rebuilt as conj(r0 x r1)), as in FP32.  The
-// rebuilt rows differ from explicit products by the links' distance from SU(3), ~1e-15 in FP64,
-// inside the 1e-12 parity bound.
-#ifndef QCB_CLOVER64_ROWS
-#define QCB_CLOVER64_ROWS 1
 #endif
 
 // ------------------------------------------------------------------ heatbath
@@ -1331,28 +1325,56 @@ __device__ __forceinline__ M3<R> from_rows(const Cx<R> r[2][3]) {
 // One clover leaf A' B' C' D' (' = adjoint where the flag is set), in the reference's association
 // ((A' B') C') D'.  The first two rows are carried through the three products and the third row
 // of the SU(3) leaf is rebuilt (60 instead of 81 complex multiply-adds; the rebuilt row differs
-// from the product by the links' distance from SU(3): ~1e-15 in FP64, the FP32 rounding level in
-// FP32).  With QCB_CLOVER64_ROWS = 0, FP64 multiplies full matrices.
+// from the product by the links' distance from SU(3), the FP32 rounding level).
 template <typename R, bool DA, bool DB, bool DC, bool DD>
 __device__ __forceinline__ M3<R> clover_leaf(const M3<R>& A, const M3<R>& B, const M3<R>& C, const M3<R>& D) {
-    if constexpr (sizeof(R) == 4 || QCB_CLOVER64_ROWS) {
-        Cx<R> r[2][3];
-        link_row<R, DA>(A, 0, r[0]);
-        link_row<R, DA>(A, 1, r[1]);
-        rows_mul<R, DB>(r, B);
-        rows_mul<R, DC>(r, C);
-        rows_mul<R, DD>(r, D);
-        return from_rows(r);
-    } else {
-        const M3<R> a = DA ? adjoint(A) : A;
-        M3<R> t = DB ? mul_na(a, B) : mul_nn(a, B);
-        t = DC ? mul_na(t, C) : mul_nn(t, C);
-        return DD ? mul_na(t, D) : mul_nn(t, D);
+    Cx<R> r[2][3];
+    link_row<R, DA>(A, 0, r[0]);
+    link_row<R, DA>(A, 1, r[1]);
+    rows_mul<R, DB>(r, B);
+    rows_mul<R, DC>(r, C);
+    rows_mul<R, DD>(r, D);
+    return from_rows(r);
+}
+
+// A' B^dag C' (' = adjoint where the flag is set) by the two-row products above.
+template <typename R, bool DA, bool DC>
+__device__ __forceinline__ M3<R> clover_staple(const M3<R>& A, const M3<R>& B, const M3<R>& C) {
+    Cx<R> r[2][3];
+    link_row<R, DA>(A, 0, r[0]);
+    link_row<R, DA>(A, 1, r[1]);
+    rows_mul<R, true>(r, B);
+    rows_mul<R, DC>(r, C);
+    return from_rows(r);
+}
+// clover_acc of A B, forming only the entries that it reads.
+template <typename R>
+__device__ __forceinline__ void clover_acc_product(CloverF<R>& S, const M3<R>& A, const M3<R>& B) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            S.d[i] = fma(A(i, k).re, B(k, i).im, fma(A(i, k).im, B(k, i).re, S.d[i]));
+#pragma unroll
+        for (int j = i + 1; j < 3; j++) {
+            Cx<R> u = mkc<R>(0, 0), l = mkc<R>(0, 0);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                cmac(u, A(i, k), B(k, j));
+                cmac(l, A(j, k), B(k, i));
+            }
+            S.o[i + j - 1] = S.o[i + j - 1] + (u - cconj(l));
+        }
     }
 }
 
-// F of plane (mu, nu) at site x with the four leaves in the reference's order; also returns
-// Re Tr of leaf 1, which is the plaquette U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag.
+// F of plane (mu, nu) at site x; also returns Re Tr of leaf 1, which is the plaquette
+// U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag.  FP32 adds the four leaves in the reference's order.
+// FP64 uses that F sees L and -L^dag alike: leaf 4 enters as -(U_mu(x) S_4) beside leaf 1 = U_mu(x) S_1, leaf 3
+// as -(S_3 V) beside leaf 2 = S_2 V, V = U_mu(x-mu), so each pair costs one last product, of which only what
+// F reads is formed: 218 complex multiply-adds a plane instead of 240, 14 links loaded instead of 16.  The
+// pass is bound by FP64 chains at 8 warps an SM: 32^4 604 us against 617 (a call 675 against 707), 16^4 46.7
+// against 49.2, 12 reals level (687 against 689); at 3 blocks an SM it spills (635).
 template <typename R, int NE>
 __device__ __forceinline__ CloverF<R> clover_F(const LinkField<R, NE>& U, const Steps& st, int lex, int par, int mu,
                                                int nu, R& plaq_tr) {
@@ -1370,24 +1392,47 @@ __device__ __forceinline__ CloverF<R> clover_F(const LinkField<R, NE>& U, const 
         S.o[k] = mkc<R>(0, 0);
         S.d[k] = R(0);
     }
-    M3<R> L;
-    // leaf 1: U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag
-    L = clover_leaf<R, false, false, true, true>(U.load_ro(mu, par, h), U.load_ro(nu, opp, xpmu >> 1),
-                                                 U.load_ro(mu, opp, xpnu >> 1), U.load_ro(nu, par, h));
-    plaq_tr = (L(0, 0).re + L(1, 1).re) + L(2, 2).re;
-    clover_acc(S, L);
-    // leaf 2: U_nu(x) U_mu(x-mu+nu)^dag U_nu(x-mu)^dag U_mu(x-mu)
-    L = clover_leaf<R, false, true, true, false>(U.load_ro(nu, par, h), U.load_ro(mu, par, xmmupnu >> 1),
-                                                 U.load_ro(nu, opp, xmmu >> 1), U.load_ro(mu, opp, xmmu >> 1));
-    clover_acc(S, L);
-    // leaf 3: U_mu(x-mu)^dag U_nu(x-mu-nu)^dag U_mu(x-mu-nu) U_nu(x-nu)
-    L = clover_leaf<R, true, true, false, false>(U.load_ro(mu, opp, xmmu >> 1), U.load_ro(nu, par, xmmumnu >> 1),
-                                                 U.load_ro(mu, par, xmmumnu >> 1), U.load_ro(nu, opp, xmnu >> 1));
-    clover_acc(S, L);
-    // leaf 4: U_nu(x-nu)^dag U_mu(x-nu) U_nu(x+mu-nu) U_mu(x)^dag
-    L = clover_leaf<R, true, false, false, true>(U.load_ro(nu, opp, xmnu >> 1), U.load_ro(mu, opp, xmnu >> 1),
-                                                 U.load_ro(nu, par, xpmumnu >> 1), U.load_ro(mu, par, h));
-    clover_acc(S, L);
+    if constexpr (sizeof(R) == 8) {
+        M3<R> D = clover_staple<R, false, true>(U.load_ro(nu, opp, xpmu >> 1), U.load_ro(mu, opp, xpnu >> 1),
+                                                U.load_ro(nu, par, h));
+        const M3<R> u = U.load_ro(mu, par, h);
+        plaq_tr = R(0);
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) plaq_tr = fma(u(i, k).re, D(k, i).re, fma(-u(i, k).im, D(k, i).im, plaq_tr));
+        M3<R> B = clover_staple<R, true, false>(U.load_ro(nu, par, xpmumnu >> 1), U.load_ro(mu, opp, xmnu >> 1),
+                                                U.load_ro(nu, opp, xmnu >> 1));
+#pragma unroll
+        for (int k = 0; k < 9; k++) D.e[k] = D.e[k] - B.e[k];
+        clover_acc_product(S, u, D);
+        D = clover_staple<R, false, true>(U.load_ro(nu, par, h), U.load_ro(mu, par, xmmupnu >> 1),
+                                          U.load_ro(nu, opp, xmmu >> 1));
+        B = clover_staple<R, true, false>(U.load_ro(nu, opp, xmnu >> 1), U.load_ro(mu, par, xmmumnu >> 1),
+                                          U.load_ro(nu, par, xmmumnu >> 1));
+#pragma unroll
+        for (int k = 0; k < 9; k++) D.e[k] = D.e[k] - B.e[k];
+        clover_acc_product(S, D, U.load_ro(mu, opp, xmmu >> 1));
+    } else {
+        M3<R> L;
+        // leaf 1: U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag
+        L = clover_leaf<R, false, false, true, true>(U.load_ro(mu, par, h), U.load_ro(nu, opp, xpmu >> 1),
+                                                     U.load_ro(mu, opp, xpnu >> 1), U.load_ro(nu, par, h));
+        plaq_tr = (L(0, 0).re + L(1, 1).re) + L(2, 2).re;
+        clover_acc(S, L);
+        // leaf 2: U_nu(x) U_mu(x-mu+nu)^dag U_nu(x-mu)^dag U_mu(x-mu)
+        L = clover_leaf<R, false, true, true, false>(U.load_ro(nu, par, h), U.load_ro(mu, par, xmmupnu >> 1),
+                                                     U.load_ro(nu, opp, xmmu >> 1), U.load_ro(mu, opp, xmmu >> 1));
+        clover_acc(S, L);
+        // leaf 3: U_mu(x-mu)^dag U_nu(x-mu-nu)^dag U_mu(x-mu-nu) U_nu(x-nu)
+        L = clover_leaf<R, true, true, false, false>(U.load_ro(mu, opp, xmmu >> 1), U.load_ro(nu, par, xmmumnu >> 1),
+                                                     U.load_ro(mu, par, xmmumnu >> 1), U.load_ro(nu, opp, xmnu >> 1));
+        clover_acc(S, L);
+        // leaf 4: U_nu(x-nu)^dag U_mu(x-nu) U_nu(x+mu-nu) U_mu(x)^dag
+        L = clover_leaf<R, true, false, false, true>(U.load_ro(nu, opp, xmnu >> 1), U.load_ro(mu, opp, xmnu >> 1),
+                                                     U.load_ro(nu, par, xpmumnu >> 1), U.load_ro(mu, par, h));
+        clover_acc(S, L);
+    }
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         S.o[k] = scl((R)0.125, S.o[k]);
