@@ -405,8 +405,7 @@ int field_new(const int L[4], int prec, int store, cudaStream_t stream, qcb_fiel
 }  // namespace
 
 // Deterministic final reduction (one block, fixed summation order for a given nb).
-__global__ void qcb::k_finalize(const double* __restrict__ partials, int nb, int nv, unsigned max_mask, double* out,
-                                int* row) {
+__global__ void qcb::k_finalize(const double* partials, int nb, int nv, unsigned max_mask, double* out, int* row) {
     __shared__ double sm[4 * kFinalizeThreads];
     const int k = threadIdx.x / kFinalizeThreads, t = threadIdx.x % kFinalizeThreads;
     const bool ismax = (max_mask >> k) & 1u;

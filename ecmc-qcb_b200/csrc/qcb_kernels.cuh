@@ -1193,8 +1193,7 @@ __device__ __forceinline__ void block_sum_store(double v[NV], double* partials, 
 // fixed order).  Bit k of max_mask set: component k is a max instead of a sum.  Into out[0..nv), or
 // with a row counter into row *row of out, which then advances.
 constexpr int kFinalizeThreads = 256;
-__global__ void k_finalize(const double* __restrict__ partials, int nb, int nv, unsigned max_mask, double* out,
-                           int* row);
+__global__ void k_finalize(const double* partials, int nb, int nv, unsigned max_mask, double* out, int* row);
 
 // Plaquette (observables_mpi.cpp:11-35): per site sum over mu<nu of Re Tr(U_mu(x) U_nu(x+mu)
 // U_mu(x+nu)^dag U_nu(x)^dag)/3, evaluated as Re Tr((U_mu(x) U_nu(x+mu)) (U_nu(x) U_mu(x+nu))^dag).

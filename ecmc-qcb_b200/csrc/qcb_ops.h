@@ -12,7 +12,9 @@ namespace qcb {
 
 // Launch of a kernel that begins with work of its own and then waits for the launches before it
 // (cudaGridDependencySynchronize): its blocks may start when those of the previous launch have
-// ended or have said that they may, without the gap between two launches in a stream.
+// ended or have said that they may, without the gap between two launches in a stream.  The launch
+// before may still be writing while such a kernel runs, so what it writes is read as ordinary memory: no
+// const __restrict__ parameter, __ldg or load_ro, which promise that nobody writes it meanwhile.
 template <typename... P, typename... A>
 inline cudaError_t launch_early(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, A... a) {
     cudaLaunchConfig_t cfg = {};
