@@ -26,7 +26,10 @@ inline cudaError_t launch_early(void (*k)(P...), unsigned grid, unsigned block, 
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
+    // a refused launch is reported here and not left for the check after the next one
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 // A work list of tiles over device-resident lattice descriptors.

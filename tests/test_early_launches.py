@@ -6,10 +6,11 @@ the read-only path, whose contract is that nobody writes the memory during the k
 import glob
 import os
 import re
+import subprocess
 
 import pytest
 
-from conftest import PKG_DIR
+from conftest import PKG_DIR, ROOT
 
 CSRC = os.path.join(PKG_DIR, "csrc")
 TEXT = {os.path.basename(p): re.sub(r"//[^\n]*", "", open(p).read())
@@ -55,3 +56,13 @@ def test_early_kernel_reads_ordinary_memory(name):
     params, body = definition(name)
     assert "__restrict__" not in params
     assert "__ldg" not in body and "load_ro" not in body
+
+
+@pytest.mark.gpu
+def test_a_refused_launch_leaves_no_error_behind(tmp_path):
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    exe = str(tmp_path / "early_error")
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-ccbin", "/usr/bin/g++",
+                    "-I" + CSRC, os.path.join(ROOT, "tests", "cpp", "early_error.cu"), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
