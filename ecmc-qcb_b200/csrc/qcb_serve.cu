@@ -34,6 +34,7 @@
 #include <thread>
 #include <vector>
 
+#include "qcb_hostbuf.h"
 #include "qcb_internal.h"
 #include "qcb_ops.h"
 
@@ -48,19 +49,14 @@ using namespace qcb;
 
 namespace {
 
-// A request's links on the host between its submission and its admission, in the server's format (its
-// precision, and the stored rows only): half to a sixth of the caller's FP64 links.
-struct HostBuf {
-    void* p = nullptr;
-    size_t cap = 0;
-};
-
 struct Request {
     uint64_t id = 0;
     Geom g{};
     double eps = 0.02;
     int n_steps = 1;
-    HostBuf input;  // links, given back after their upload
+    // its links on the host between its submission and its admission, in the server's format (its precision, and
+    // the stored rows only): half to a sixth of the caller's FP64 links; given back after their upload
+    HostBuf input;
     std::vector<double> tqe;    // 3 * n_steps results
     double t_submit = 0, t_admit = 0, t_done = 0;
     void* buf = nullptr;  // W, W', Z, measurements in one allocation
@@ -82,6 +78,9 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr int64_t kBigVh = (int64_t)1 << 17;
 bool is_big(const Request* r) { return r->g.Vh >= kBigVh; }
 
+// Bytes of request links' buffers that a server keeps for later requests, at most.
+constexpr size_t kHostPoolBytes = (size_t)1 << 30;
+
 }  // namespace
 
 struct qcb_server_s {
@@ -91,9 +90,7 @@ struct qcb_server_s {
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
     std::deque<Request*> pending, done;
-    // host buffers that wait for another request (under mu), at most kHostPoolBytes of them
-    std::vector<HostBuf> host_free;
-    size_t host_free_bytes = 0;
+    HostBufs host{kHostPoolBytes};  // buffers of the requests' links
     std::vector<Request*> active;
     std::vector<Request*> small, big;  // the active set split by size (rebuild)
     double* big_partials = nullptr;
@@ -212,47 +209,7 @@ bool grow(qcb_server_s* s, T** p, size_t* cap, size_t n) {
 // eight requests of 8^4 to 24^4 with 50 measured steps 52 ms instead of 171 (a new server's first 65, not 186).
 // The buffers stay ordinary memory: page-locking them made the steady state 10 ms shorter, but locking
 // 150 MB beside a running scheduler took a new server's first requests up to 0.9 s.
-constexpr size_t kHostPoolBytes = (size_t)1 << 30;
 constexpr size_t kSplitBytes = (size_t)4 << 20;  // input of a submission beyond which threads share it
-
-// A buffer of at least n bytes (p = NULL: out of memory): the smallest free one that does, unless it is
-// more than four times as large, or a new one.
-HostBuf take_buf(qcb_server_s* s, size_t n) {
-    HostBuf b;
-    {
-        std::lock_guard<std::mutex> lk(s->mu);
-        size_t best = s->host_free.size();
-        for (size_t i = 0; i < s->host_free.size(); i++) {
-            const size_t cap = s->host_free[i].cap;
-            if (cap >= n && cap / 4 <= n && (best == s->host_free.size() || cap < s->host_free[best].cap)) best = i;
-        }
-        if (best < s->host_free.size()) {
-            b = s->host_free[best];
-            s->host_free.erase(s->host_free.begin() + (long)best);
-            s->host_free_bytes -= b.cap;
-            return b;
-        }
-    }
-    b.p = malloc(n);
-    b.cap = n;
-    return b;
-}
-
-// Back to the free ones; the oldest leave where they would hold more than kHostPoolBytes.
-void give_buf(qcb_server_s* s, HostBuf b) {
-    std::vector<HostBuf> out;
-    {
-        std::lock_guard<std::mutex> lk(s->mu);
-        s->host_free.push_back(b);
-        s->host_free_bytes += b.cap;
-        while (s->host_free_bytes > kHostPoolBytes) {
-            out.push_back(s->host_free.front());
-            s->host_free_bytes -= out.back().cap;
-            s->host_free.erase(s->host_free.begin());
-        }
-    }
-    for (HostBuf& o : out) free(o.p);
-}
 
 // Reals of links [a, b) of FP64 AoS links, rounded to T; ne complexes of each link.
 template <typename T>
@@ -348,7 +305,7 @@ bool admit(qcb_server_s* s, Request* r) {
     note_launches(1);
     if (!cuda_ok(s, cudaEventRecord(s->ev_layout, r->st), "layout event")) return false;
     s->layout_pending = true;
-    give_buf(s, r->input);
+    s->host.give(r->input);
     r->input = HostBuf{};
     r->tick0 = is_big(r) ? s->tick_b : s->tick;
     r->flip = (int)((is_big(r) ? s->nflow_b : s->nflow) & 1);  // current links in buffer A
@@ -718,7 +675,6 @@ int qcb_serve_destroy(qcb_server s) {
         delete r;
     }
     for (Request* r : s->done) delete r;
-    for (HostBuf& b : s->host_free) free(b.p);
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->stream_small) cudaStreamSynchronize(s->stream_small);
     if (s->ev_layout) cudaEventDestroy(s->ev_layout);
@@ -771,7 +727,7 @@ int qcb_serve_submit(qcb_server s, uint64_t id, const int L[4], const double* li
         delete r;
         return fail(QCB_ENOMEM, "serve submit: request needs %zu bytes, budget is %zu", need, s->budget);
     }
-    r->input = take_buf(s, packed_bytes(s->fmt, V));
+    r->input = s->host.take(packed_bytes(s->fmt, V));
     if (!r->input.p) {
         delete r;
         return fail(QCB_ENOMEM, "host allocation");

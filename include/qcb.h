@@ -275,7 +275,9 @@ int qcb_batch_tune(qcb_batch b, int n_hits, int n_trial, int allow_store_change,
  * max_active <= 0: no limit besides the budget.  Every request takes its measurements from
  * measuring RK3 stage 1 launches, as qcb_flow_measure does; a request below 2^17 half-sites holds
  * 114 reals a site for them within its memory, and for the larger ones, which run alone, the server
- * keeps scratch outside the budget: 114 reals a site of the largest, in the server's precision. */
+ * keeps scratch outside the budget: 114 reals a site of the largest, in the server's precision.  The
+ * server also keeps the host buffers of its copies of the requests' links for later requests, at most
+ * 1 GiB of them together (a larger one is freed after its upload), until it is destroyed. */
 int qcb_serve_create(size_t hbm_budget_bytes, int prec, int store, int n_rk, int max_active, qcb_server* out);
 int qcb_serve_destroy(qcb_server s);
 /* Server options.  QCB_SERVE_GRAPHS (default 1): while the resident set of small requests is
@@ -288,7 +290,9 @@ int qcb_serve_set_option(qcb_server s, int option, int value);
 /* Seconds on the server's clock (the clock of the times returned by qcb_serve_poll). */
 double qcb_serve_now(qcb_server s);
 /* Queues one request (thread-safe): host AoS FP64 links of an L[0..3] lattice, flow step eps,
- * n_steps measurements at t = 0, n_rk*eps, ... (n_steps - 1 flow blocks).  The links are copied. */
+ * n_steps measurements at t = 0, n_rk*eps, ... (n_steps - 1 flow blocks).  The links are copied, rounded to
+ * the server's format, before the call returns; for more than 4 MiB of them up to three threads of
+ * the call's own help. */
 int qcb_serve_submit(qcb_server s, uint64_t id, const int L[4], const double* links, double eps, int n_steps);
 /* Pops one completed request: returns 1 and fills id, tQE (3 * min(max_steps, n_steps) doubles:
  * t, Q, E), n_steps and times[3] = (submitted, admitted, completed); returns 0 if none is ready. */
