@@ -1,4 +1,8 @@
-// qcb_hostbuf.h -- host buffers that are used again (the server's copies of the requests' links).  Plain C++.
+// qcb_hostbuf.h -- host buffers that are used again, and wait for the end of a copy before that.
+//
+// A server takes a buffer for each request's links, fills it, starts a copy from it to the device and gives
+// it back with the event that follows the copy.  Another thread may fill a buffer the moment it takes it,
+// so one whose copy has not ended is never handed out.  Plain C++: Event is a cudaEvent_t in the server.
 #pragma once
 #include <stdlib.h>
 
@@ -12,6 +16,7 @@ struct HostBuf {
     size_t cap = 0;
 };
 
+template <class Event>
 class HostBufs {
   public:
     // At most `limit` bytes wait for another use.
@@ -20,6 +25,7 @@ class HostBufs {
     HostBufs& operator=(const HostBufs&) = delete;
     ~HostBufs() {
         for (HostBuf& b : free_) free(b.p);
+        for (Copy& c : copies_) free(c.b.p);
     }
 
     // A buffer of at least n bytes (p = NULL: out of memory): the smallest free one that does, unless it is
@@ -65,6 +71,34 @@ class HostBufs {
         }
     }
 
+    // Back once the copy that `done` follows has ended.  False without memory to note it: b stays the caller's.
+    bool give_after(HostBuf b, Event done) {
+        std::lock_guard<std::mutex> lk(mu_);
+        try {
+            copies_.push_back(Copy{b, done});
+        } catch (...) {
+            return false;
+        }
+        return true;
+    }
+    // Gives back the buffers whose event `ended` finds complete, and hands each such event to `release`.
+    template <class Ended, class Release>
+    void reclaim(Ended ended, Release release) {
+        for (;;) {
+            Copy c;
+            {
+                std::lock_guard<std::mutex> lk(mu_);
+                size_t i = 0;
+                while (i < copies_.size() && !ended(copies_[i].done)) i++;
+                if (i == copies_.size()) return;
+                c = copies_[i];
+                copies_.erase(copies_.begin() + (long)i);
+            }
+            release(c.done);
+            give(c.b);
+        }
+    }
+
   private:
     bool keep(HostBuf b) {
         std::lock_guard<std::mutex> lk(mu_);
@@ -76,10 +110,15 @@ class HostBufs {
         bytes_ += b.cap;
         return true;
     }
+    struct Copy {
+        HostBuf b;
+        Event done;
+    };
     const size_t limit_;
     std::mutex mu_;
     std::vector<HostBuf> free_;
     size_t bytes_ = 0;
+    std::vector<Copy> copies_;
 };
 
 }  // namespace qcb

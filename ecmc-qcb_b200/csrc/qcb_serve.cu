@@ -90,7 +90,7 @@ struct qcb_server_s {
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
     std::deque<Request*> pending, done;
-    HostBufs host{kHostPoolBytes};  // buffers of the requests' links
+    HostBufs<cudaEvent_t> host{kHostPoolBytes};  // buffers of the requests' links
     std::vector<Request*> active;
     std::vector<Request*> small, big;  // the active set split by size (rebuild)
     double* big_partials = nullptr;
@@ -298,18 +298,35 @@ bool admit(qcb_server_s* s, Request* r) {
     const size_t nb = packed_bytes(s->fmt, r->g.V);
     if (!grow(s, &s->staging, &s->staging_cap, (nb + sizeof(double2) - 1) / sizeof(double2))) return false;
     if (s->layout_pending && !cuda_ok(s, cudaStreamWaitEvent(r->st, s->ev_layout, 0), "upload order")) return false;
-    // pageable source: it has been read when the call returns
     if (!cuda_ok(s, cudaMemcpyAsync(s->staging, r->input.p, nb, cudaMemcpyHostToDevice, r->st), "request upload"))
         return false;
+    // another submission may fill the buffer as soon as it is back: not before the copy from it has ended
+    cudaEvent_t copied;
+    if (!cuda_ok(s, cudaEventCreateWithFlags(&copied, cudaEventDisableTiming), "upload event")) return false;
+    const bool noted = cuda_ok(s, cudaEventRecord(copied, r->st), "upload event");
+    if (noted && s->host.give_after(r->input, copied))
+        r->input = HostBuf{};
+    else
+        cudaEventDestroy(copied);  // the request keeps its buffer to its end
+    if (!noted) return false;
     if (!cuda_ok(s, fmt_ops(s->fmt).packed_to_soa(r->g, s->staging, r->buf, r->st), "request layout")) return false;
     note_launches(1);
     if (!cuda_ok(s, cudaEventRecord(s->ev_layout, r->st), "layout event")) return false;
     s->layout_pending = true;
-    s->host.give(r->input);
-    r->input = HostBuf{};
     r->tick0 = is_big(r) ? s->tick_b : s->tick;
     r->flip = (int)((is_big(r) ? s->nflow_b : s->nflow) & 1);  // current links in buffer A
     return true;
+}
+
+// The buffers whose uploads have ended, back for other requests.
+void reclaim_buffers(qcb_server_s* s) {
+    s->host.reclaim(
+        [](cudaEvent_t e) {
+            if (cudaEventQuery(e) != cudaErrorNotReady) return true;
+            cudaGetLastError();  // not an error: the next launch's check must not see it
+            return false;
+        },
+        [](cudaEvent_t e) { cudaEventDestroy(e); });
 }
 
 bool finish(qcb_server_s* s, Request* r) {
@@ -320,6 +337,8 @@ bool finish(qcb_server_s* s, Request* r) {
     if (!cuda_ok(s, cudaFreeAsync(r->buf, r->st), "request free")) return false;
     if (!cuda_ok(s, cudaStreamSynchronize(r->st), "result sync")) return false;
     r->buf = nullptr;
+    if (r->input.p) s->host.give(r->input);
+    r->input = HostBuf{};
     r->tqe.resize((size_t)r->n_steps * 3);
     double t = 0.0;
     for (int k = 0; k < r->n_steps; k++) {
@@ -588,6 +607,7 @@ void scheduler(qcb_server_s* s) {
         for (Request* r : fresh) {
             ok = ok && admit(s, r);
             s->active.push_back(r);
+            reclaim_buffers(s);
         }
         if (ok && !fresh.empty()) ok = rebuild(s);
         if (!ok) break;
@@ -598,6 +618,7 @@ void scheduler(qcb_server_s* s) {
         if (!s->big.empty()) ok = big_tick(s, rep);
         for (int j = 0; ok && j < m && !s->small.empty(); j++) ok = small_tick(s, rep);
         if (!ok) break;
+        reclaim_buffers(s);
         {
             std::lock_guard<std::mutex> lk(s->mu);
             s->ticks++;
@@ -607,6 +628,7 @@ void scheduler(qcb_server_s* s) {
     }
     cudaStreamSynchronize(s->stream);
     cudaStreamSynchronize(s->stream_small);
+    reclaim_buffers(s);
     drop_tick_graphs(s);
 }
 

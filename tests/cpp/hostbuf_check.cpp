@@ -1,4 +1,4 @@
-// The server's reuse of host buffers (qcb_hostbuf.h): which buffer a request gets, and what is kept.
+// The server's reuse of host buffers (qcb_hostbuf.h): which buffer a request gets and when, and what is kept.
 #include <stdio.h>
 
 #include "qcb_hostbuf.h"
@@ -14,7 +14,7 @@ static void expect(bool ok, const char* what) {
 
 // a buffer above the limit is freed; those that wait stay
 static void above_the_limit() {
-    HostBufs h(1000);
+    HostBufs<int> h(1000);
     const HostBuf a = h.take(300), b = h.take(400), big = h.take(1500);
     h.give(a);
     h.give(b);
@@ -27,7 +27,7 @@ static void above_the_limit() {
 
 // at the limit the oldest leave
 static void at_the_limit() {
-    HostBufs h(1000);
+    HostBufs<int> h(1000);
     const HostBuf a = h.take(300), b = h.take(400), c = h.take(600);
     h.give(a);
     h.give(b);
@@ -43,7 +43,7 @@ static void at_the_limit() {
 
 // the smallest that is large enough, but none of more than four times the size
 static void choice() {
-    HostBufs h(1 << 20);
+    HostBufs<int> h(1 << 20);
     const HostBuf a = h.take(100), b = h.take(200), c = h.take(4000);
     h.give(c);
     h.give(b);
@@ -56,7 +56,30 @@ static void choice() {
     h.give(z);
 }
 
+// a buffer whose copy has not ended is not handed out
+static void copies() {
+    HostBufs<int> h(1000);
+    const HostBuf a = h.take(300), b = h.take(300);
+    expect(h.give_after(a, 1) && h.give_after(b, 2), "noted");
+    int released = 0;
+    auto release = [&](int e) { released |= e; };
+    h.reclaim([](int) { return false; }, release);
+    const HostBuf x = h.take(290);
+    expect(x.cap == 290 && released == 0, "a buffer handed out while a copy reads it");
+    h.reclaim([](int e) { return e == 2; }, release);
+    const HostBuf y = h.take(290);
+    expect(y.p == b.p && released == 2, "the buffer whose copy has ended, and its event alone");
+    h.reclaim([](int) { return true; }, release);
+    const HostBuf z = h.take(290);
+    expect(z.p == a.p && released == 3, "the other one after its copy");
+    h.give(x);
+    h.give(y);
+    h.give(z);
+    expect(h.give_after(h.take(50), 4), "noted");  // a copy not reclaimed: freed with the class
+}
+
 int main() {
+    copies();
     above_the_limit();
     at_the_limit();
     choice();
