@@ -1055,6 +1055,7 @@ __device__ __forceinline__ void flow_link(const Geom& g, const LinkField<R, NE>&
 // of the sectors and a stage takes 649-660 against 695 us (24^4: 185 against 190).  FP32 kernels, bound
 // by issue, keep one class a block (blockIdx.x = 8 * site block + mu * 2 + parity): the direction is
 // then uniform over the block (16^4: 30.6 against 31.6 us).
+static_assert(QCB_FLOW_THREADS == 128, "flow_map: four warps a block, and the work lists' tiles of 128 half-sites");
 template <typename R>
 __device__ __forceinline__ void flow_map(unsigned b, int& mu, int& par, int64_t& h) {
     if constexpr (sizeof(R) == 8) {
