@@ -62,7 +62,7 @@ struct FmtImpl {
         if constexpr (sizeof(R) == 8)
             if (g.Vh <= kHbGroupMaxVh)
                 return launch_early(k_hb_group<NE, MU>, (unsigned)((g.Vh + kHbGroupLinks - 1) / kHbGroupLinks),
-                                    kHbLanes * kHbGroupLinks, s, g, view(links, g.Vh), par, c_alpha, n_hits, seed,
+                                    kHbGroupThreads, s, g, view(links, g.Vh), par, c_alpha, n_hits, seed,
                                     sweep, rep, err);
         const unsigned nb = (unsigned)((g.Vh + QCB_HB_THREADS - 1) / QCB_HB_THREADS);
         return launch_early(k_hb_subsweep<R, NE, MU>, nb, QCB_HB_THREADS, s, g, view(links, g.Vh), par, c_alpha, n_hits,

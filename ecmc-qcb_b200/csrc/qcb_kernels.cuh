@@ -781,7 +781,9 @@ struct HbSlotFits {
 // and are formed before the wait for it.  The permission for the next launch is left to the blocks' ends
 // (given at their start or after the hits, the next launch's blocks crowd onto the SMs with room: a 16^4
 // sweep 252 and 181 us, at the ends 164).  A sweep at N_hits = 2: 12^4 148 to 133 us, 16^4 181 to 164, a
-// 131 k-site lattice 283 to 271; 24^4 and above 0-3%.
+// 131 k-site lattice 283 to 271; 24^4 and above 0-3%.  Chains side by side that overfill the GPU give part of
+// it back, since a block holds its place while it waits: four of 16^4 430 against 415 us, four of 24^4 1867 against
+// 1841, sixteen of 12^3 x 8 463 against 477.
 template <typename R, int NE, int MU>
 __global__ void __launch_bounds__(QCB_HB_THREADS, QCB_HB_MINB(R))
     k_hb_subsweep(Geom g, LinkField<R, NE> U, int par, double c_alpha, int n_hits, uint64_t seed, uint32_t sweep,
@@ -794,81 +796,87 @@ __global__ void __launch_bounds__(QCB_HB_THREADS, QCB_HB_MINB(R))
                                    slot + threadIdx.x, QCB_HB_THREADS);
 }
 
-// Heatbath sub-sweep of a small lattice (FP64): eight lanes a link, 16 links a block.  With one thread a
-// link, an 8^4 set is 64 warps on 148 SMs and a launch lasts as long as one link's serial chain (18 us:
-// three rounds of staple loads, then 6 subgroup updates of Philox calls, logarithms and a sine/cosine
-// each).  What does not depend on the updates in sequence is spread over the lanes:
-//   * the draws of the link's stream, whatever the attempts turn out to be: for every Philox call m its
-//     two uniforms, the attempt at m (log r1 + cos^2(2 pi r2) log r3 and delta^2, from calls m and
-//     m + 1) and the direction that call m would give (kp_fill).  They need no link, so they
-//     run before the wait for the previous launch and overlap its tail (with that and the
-//     permission to start given at the top, 83 to 68 us an 8^4 sweep);
+// Heatbath sub-sweep of a small lattice (FP64): 16 links a block of four warps.  With one thread a link, an 8^4
+// set is 64 warps on 148 SMs and a launch lasts as long as one link's serial chain (16 us: three rounds of
+// staple loads, then 6 subgroup updates of Philox calls, logarithms and a sine/cosine each).  What does not
+// depend on the updates in sequence is spread over the block:
+//   * the draws of the links' streams, whatever the attempts turn out to be: for each of the next 24 Philox
+//     calls m the attempt at m (log r1 + cos^2(2 pi r2) log r3 and delta^2, from calls m and m + 1) and the
+//     direction that call m would give.  They need no link, so they run before the wait for the
+//     previous launch, beside its updates;
 //   * the six staples, forward ones by warps 0-1 and backward ones by warps 2-3.
-// The updates run on the eight lanes alike, from registers.  Every value is formed by the operations of
-// k_hb_subsweep in their order: same links, bit for bit.  A sweep at N_hits = 2 (1): 4^4 44 (34) us
-// against 117 (81) with one thread a link, 8^4 68 (46) against 126 (87), 12^3 x 8 80 (54) against
-// 134 (95); past one wave of blocks (3 a SM: 7104 links) it is no faster (12^4 130 against 133, 16^4 353
-// against 164), which is where kHbGroupMaxVh lies.
-struct KPDraw {
-    double log_term, delta2;
-    KPDir dir;
+// Half a warp then runs the updates from the table, one lane a link; an attempt past the table is drawn on
+// the spot, out of line, and every two hits the block fills the table again.  Every value is formed by
+// the operations of k_hb_subsweep in their order: same links, bit for bit.
+// The next launch may start once the staples are there, so no more than one launch of a chain waits on
+// places that another chain could use.  A sweep at N_hits = 2 (1): 4^4 44 (31) us against 115 (79) with one thread
+// a link, 8^4 50 (35) against 126 (87), 12 x 8^2 x 6 51 (37) against 129 (91).
+constexpr int kHbGroupLinks = 16, kHbGroupThreads = 128;
+// The line: one block a SM.  One chain would gain beyond it (10^4: 62 against 131 us), but a link takes twice the
+// SM time of k_hb_subsweep, which chains side by side on their own streams pay once they fill the GPU.  With
+// sweeps issued by the host (18 us each) chains below the line never do: 8, 16 and 32 of 8^4 take 152, 308 and
+// 633 us a round, 167, 315 and 643 with one thread a link and plain launches; 8 of 10^4 would take 319
+// against 185.  Captured in one graph, 8 of 8^4 are level (130 and 131 us); 16 and 32, which a Batch sweeps better,
+// take 267 and 550 against 158 and 269.  (Eight lanes a link that all ran its updates took 182, 356 and 732.)
+constexpr int64_t kHbGroupMaxVh = 148 * kHbGroupLinks;
+constexpr int kKPUpdates = 6;  // of two hits
+constexpr int kKPTable = 24;   // stream positions held: the updates take 18 of them and 2 more a rejection
+// A block's draws, [position][link]: (log term, delta^2) of an attempt, (sin, cos) of a direction's two angles.
+struct KPTable {
+    double2 attempt[kKPTable][kHbGroupLinks], theta[kKPTable][kHbGroupLinks], phi[kKPTable][kHbGroupLinks];
 };
-constexpr int kHbLanes = 8, kHbGroupLinks = 16;
-constexpr int64_t kHbGroupMaxVh = 3 * 148 * kHbGroupLinks;
-constexpr int kKPTable = 24;  // stream positions held: 2 hits take 18 of them and 2 more a rejection
-static __device__ __noinline__ void kp_fill(uint64_t seed, uint32_t link, uint32_t sweep, uint32_t base, int count,
-                                     unsigned group, double2* raw, KPDraw* table) {
+static __device__ __noinline__ double2 kp_attempt_at(uint64_t seed, uint32_t link, uint32_t sweep, uint32_t n) {
     const LinkStream rng(seed, link, sweep, TAG_HB);
-    const int lane = threadIdx.x & (kHbLanes - 1);
-    __syncwarp(group);  // the old entries have been read
-    for (int m = lane; m < count; m += kHbLanes) raw[m] = rng.call(base + (uint32_t)m);
-    __syncwarp(group);
-    for (int m = lane; m < count; m += kHbLanes) {
-        const double2 P = raw[m];
-        KPDraw d;
-        d.dir = kp_direction(P);
-        d.log_term = 0.0;
-        if (m + 1 < count) {
-            const double2 Q = raw[m + 1];
-            d.log_term = kp_log(P.y, Q.x, Q.y);
-        }
-        d.delta2 = __dmul_rn(P.x, P.x);
-        table[m] = d;
-    }
-    __syncwarp(group);
+    const double2 P = rng.call(n), Q = rng.call(n + 1u);
+    return make_double2(kp_log(P.y, Q.x, Q.y), __dmul_rn(P.x, P.x));
+}
+static __device__ __noinline__ KPDir kp_direction_at(uint64_t seed, uint32_t link, uint32_t sweep, uint32_t n) {
+    return kp_direction(LinkStream(seed, link, sweep, TAG_HB).call(n));
 }
 template <int NE, int MU>
-__global__ void __launch_bounds__(kHbLanes* kHbGroupLinks)
+__global__ void __launch_bounds__(kHbGroupThreads, 4)
     k_hb_group(Geom g, LinkField<double, NE> U, int par, double c_alpha, int n_hits, uint64_t seed, uint32_t sweep,
                int reproject, int* err) {
-    __shared__ KPDraw table_s[kHbGroupLinks][kKPTable];
-    __shared__ double2 raw_s[kHbGroupLinks][kKPTable];
-    __shared__ double2 part[6][9][kHbGroupLinks], sum[kHbGroupLinks][9];
-    cudaTriggerProgrammaticLaunchCompletion();
-    const int slot = threadIdx.x / kHbLanes;
-    const unsigned group = 0xffu << (threadIdx.x & 24);
+    __shared__ KPTable T;
+    __shared__ double2 raw[kKPTable][kHbGroupLinks];
+    __shared__ double2 part[6][9][kHbGroupLinks], sum[9][kHbGroupLinks];
+    __shared__ uint32_t pos[kHbGroupLinks];
+    const int l = threadIdx.x % kHbGroupLinks, row = threadIdx.x / kHbGroupLinks;
+    const bool updates = threadIdx.x < kHbGroupLinks;
     // links past the set repeat its last one and store nothing
-    const int64_t h0 = (int64_t)blockIdx.x * kHbGroupLinks, last = g.Vh - 1;
-    const bool live = h0 + slot <= last;
-    const int h = (int)(live ? h0 + slot : last);
+    const int64_t h0 = (int64_t)blockIdx.x * kHbGroupLinks + l;
+    const bool live = h0 < g.Vh;
+    const int h = (int)(live ? h0 : g.Vh - 1);
     int c[4];
     site_coords(g, par, (uint32_t)h, c);
-    const uint32_t link = (uint32_t)lex_of(g, c) * 4u + (uint32_t)MU;
-    KPDraw* table = table_s[slot];
-    // the subgroups' calls and room for three rejections
-    int held = n_hits < 2 ? 9 * n_hits + 6 : kKPTable;
-    kp_fill(seed, link, sweep, 0u, held, group, raw_s[slot], table);
+    const int lex = lex_of(g, c);
+    const uint32_t link = (uint32_t)lex * 4u + (uint32_t)MU;
+    const int n_sub = 3 * n_hits;
+    int held = 0;  // positions of the table
+    // the table for n updates from position base of the thread's link: their calls and room for three rejections
+    auto fill = [&](uint32_t base, int n) {
+        const LinkStream rng(seed, link, sweep, TAG_HB);
+        held = min(kKPTable, 3 * n + 6);
+        for (int m = row; m < held; m += kHbGroupThreads / kHbGroupLinks) raw[m][l] = rng.call(base + (uint32_t)m);
+        __syncthreads();
+#pragma unroll 1  // (the kernel is bound by its instructions' way to the SM: unrolled it is slower)
+        for (int m = row; m < held; m += kHbGroupThreads / kHbGroupLinks) {
+            const double2 P = raw[m][l], Q = raw[min(m + 1, held - 1)][l];
+            const KPDir d = kp_direction(P);
+            T.attempt[m][l] = make_double2(kp_log(P.y, Q.x, Q.y), __dmul_rn(P.x, P.x));
+            T.theta[m][l] = make_double2(d.st, d.ct);
+            T.phi[m][l] = make_double2(d.sp, d.cp);
+        }
+    };
+    fill(0u, min(n_sub, kKPUpdates));
     cudaGridDependencySynchronize();
     {
-        // staple task: link (threadIdx & 15), k-th nu, in the order of staple_rows_into
-        const int i = threadIdx.x & 63, k = i >> 4;
-        const bool fwd = threadIdx.x < 64;
+        // staple task: the thread's link, k-th nu, in the order of staple_rows_into
+        const int k = row & 3;
+        const bool fwd = row < 4;
         if (k < 3) {
-            const int hl = (int)(h0 + (i & 15) <= last ? h0 + (i & 15) : last);
-            int cl[4];
-            site_coords(g, par, (uint32_t)hl, cl);
-            const int lex = lex_of(g, cl), opp = par ^ 1;
-            const Steps st = make_steps(g, cl);
+            const int opp = par ^ 1;
+            const Steps st = make_steps(g, c);
             const int nu = k < MU ? k : k + 1;
             const int xmu = lex + st.up[MU], dnu = sel4(st.dn, nu), xmnu = lex + dnu;
             Cx<double> r[2][3];
@@ -920,60 +928,78 @@ __global__ void __launch_bounds__(kHbLanes* kHbGroupLinks)
             for (int j = 0; j < 3; j++) {
                 const int j1 = (j + 1) % 3, j2 = (j + 2) % 3;
                 const Cx<double> r2 = conj_cross(r[0][j1], r[1][j2], r[0][j2], r[1][j1]);
-                p[j][i & 15] = make_double2(r[0][j].re, r[0][j].im);
-                p[3 + j][i & 15] = make_double2(r[1][j].re, r[1][j].im);
-                p[6 + j][i & 15] = make_double2(r2.re, r2.im);
+                p[j][l] = make_double2(r[0][j].re, r[0][j].im);
+                p[3 + j][l] = make_double2(r[1][j].re, r[1][j].im);
+                p[6 + j][l] = make_double2(r2.re, r2.im);
             }
         }
     }
-    M3<double> u = U.load(MU, par, h);
+    M3<double> u, A;
+    if (updates) u = U.load(MU, par, h);
     __syncthreads();
-    for (int t = threadIdx.x; t < 9 * kHbGroupLinks; t += kHbLanes * kHbGroupLinks) {
-        const int e = t >> 4, l = t & 15;
+    for (int e = row; e < 9; e += kHbGroupThreads / kHbGroupLinks) {
         double2 v = make_double2(0.0, 0.0);
 #pragma unroll
         for (int s = 0; s < 6; s++) {
             v.x += part[s][e][l].x;
             v.y += part[s][e][l].y;
         }
-        sum[l][e] = v;
+        sum[e][l] = v;
     }
     __syncthreads();
-    M3<double> A;
+    cudaTriggerProgrammaticLaunchCompletion();
+    if (updates) {
 #pragma unroll
-    for (int e = 0; e < 9; e++) A.e[e] = mkc<double>(sum[slot][e].x, sum[slot][e].y);
-    uint32_t base = 0, n = 0;  // position of table[0], position of the next attempt
+        for (int e = 0; e < 9; e++) A.e[e] = mkc<double>(sum[e][l].x, sum[e][l].y);
+    }
+    uint32_t base = 0, n = 0;  // position of the table, position of the next attempt
     // su2_step with its draws from the table
     auto step = [&](const Quat& w) {
         const double ik = rsqrt(w.a0 * w.a0 + w.a1 * w.a1 + w.a2 * w.a2 + w.a3 * w.a3);
         const Quat v = {w.a0 * ik, w.a1 * ik, w.a2 * ik, w.a3 * ik};
         const double m05a = c_alpha * ik;
         const int cap = (m05a < 0.0 && isfinite(m05a)) ? KP_MAX_ATTEMPTS : 0;
-        for (int it = 0; it < cap; it++) {
-            if ((int)(n - base) > held - 3) {
-                kp_fill(seed, link, sweep, n, kKPTable, group, raw_s[slot], table);
-                base = n;
-                held = kKPTable;
-            }
-            const KPDraw* d = table + (n - base);
-            const double lsq = __dmul_rn(m05a, d->log_term);
-            if (d->delta2 <= __dadd_rn(1.0, -lsq)) {
+        for (int it = 0; it < cap; it++, n += 2u) {
+            const int m = (int)(n - base);
+            const bool in = m <= held - 3;
+            const double2 a = in ? T.attempt[m][l] : kp_attempt_at(seed, link, sweep, n);
+            const double lsq = __dmul_rn(m05a, a.x);
+            if (a.y <= __dadd_rn(1.0, -lsq)) {
+                KPDir d;
+                if (in) {
+                    const double2 th = T.theta[m + 2][l], ph = T.phi[m + 2][l];
+                    d = KPDir{th.x, th.y, ph.x, ph.y};
+                } else {
+                    d = kp_direction_at(seed, link, sweep, n + 2u);
+                }
                 n += 3u;
-                return kp_element(__dadd_rn(1.0, -__dmul_rn(2.0, lsq)), d[2].dir, v);
+                return kp_element(__dadd_rn(1.0, -__dmul_rn(2.0, lsq)), d, v);
             }
-            n += 2u;
         }
-        if ((threadIdx.x & (kHbLanes - 1)) == 0) atomicOr(err, cap > 0 ? (int)DERR_KP_CAP : (int)DERR_KP_SCALE);
+        atomicOr(err, cap > 0 ? (int)DERR_KP_CAP : (int)DERR_KP_SCALE);
         return Quat{1.0, 0.0, 0.0, 0.0};
     };
+    for (int done = 0; done < n_sub; done += kKPUpdates) {
+        if (done > 0) {
+            __syncthreads();
+            base = pos[l];
+            fill(base, min(n_sub - done, kKPUpdates));
+            __syncthreads();
+        }
+        if (updates) {
 #pragma unroll 1
-    for (int hit = 0; hit < n_hits; hit++) {
-        cm_apply<double, 0, 1>(u, step(cm_quaternion<double, 0, 1>(u, A)));
-        cm_apply<double, 1, 2>(u, step(cm_quaternion<double, 1, 2>(u, A)));
-        cm_apply<double, 0, 2>(u, step(cm_quaternion<double, 0, 2>(u, A)));
+            for (int it = done; it < min(n_sub, done + kKPUpdates); it += 3) {
+                cm_apply<double, 0, 1>(u, step(cm_quaternion<double, 0, 1>(u, A)));
+                cm_apply<double, 1, 2>(u, step(cm_quaternion<double, 1, 2>(u, A)));
+                cm_apply<double, 0, 2>(u, step(cm_quaternion<double, 0, 2>(u, A)));
+            }
+            pos[l] = n;
+        }
     }
-    if (reproject) reproject_fp64(u);
-    if (live && (threadIdx.x & (kHbLanes - 1)) == 0) U.store(MU, par, h, u);
+    if (updates) {
+        if (reproject) reproject_fp64(u);
+        if (live) U.store(MU, par, h, u);
+    }
 }
 
 // One link's heatbath update (the C ABI's single-link entry, qcb_hb_link; reference
