@@ -689,7 +689,8 @@ int qcb_field_copy(qcb_field dst, qcb_field src) {
         CK(cudaMemcpyAsync(dst->links, src->links, link_bytes(dst->fmt, dst->g.Vh), cudaMemcpyDeviceToDevice,
                            dst->stream));
     } else {
-        // (refused while a prefetched configuration waits, as every change of the links but its commit)
+        // The conversion needs no staging buffer.  The call is refused while a prefetched configuration waits in
+        // dst's because the interface says so, from when it went through that buffer; the same format is not.
         if (dst->prefetch_pending)
             return fail(QCB_EINVAL, "a prefetched configuration occupies the staging buffer: commit it first");
         RET(launch(dst, QCB_K_OTHER, [&] {

@@ -78,8 +78,8 @@ int qcb_field_download_aos(qcb_field f, double* links);
  * call after the commit has synchronised the field (qcb_field_sync, or any call that returns a
  * result); from pageable memory the copy is staged before the prefetch returns.  While a
  * prefetched configuration waits for its commit, the calls that need the staging buffer
- * (qcb_field_upload_aos / download_aos, a second prefetch, ILDG I/O, a copy between formats)
- * return QCB_EINVAL. */
+ * (qcb_field_upload_aos / download_aos, a second prefetch, ILDG I/O) and a copy into the field from
+ * another format return QCB_EINVAL; a copy within the format, sweeps and observables do not. */
 int qcb_field_prefetch_aos(qcb_field f, const double* links);
 int qcb_field_commit_prefetch(qcb_field f);
 /* Same, from / to device memory (AoS doubles already on the field's device). */
