@@ -110,7 +110,7 @@ int run_phase_set(qcb_batch_s* b, int n_hits, int variant) {
     return QCB_OK;
 }
 
-// One sweep executed eagerly (also warms the launchers' occupancy caches before a capture).
+// One sweep executed eagerly (before a capture it also loads the kernels).
 int sweep_eager(qcb_batch_s* b, int n_hits, int variant) {
     RET(run_phase_set(b, n_hits, variant));
     k_bump_sweep<<<1, 1, 0, b->stream>>>(b->d_sweep);
@@ -354,7 +354,7 @@ int qcb_batch_tune(qcb_batch b, int n_hits, int n_trial, int allow_store_change,
     double best = 1e300, times[kHbVariants + 1] = {0};
     int best_v = b->variant;
     for (int v = 0; v < kHbVariants; v++) {
-        RET(sweep_eager(b, n_hits, v));  // warm-up (and occupancy query outside the timing)
+        RET(sweep_eager(b, n_hits, v));  // warm-up
         cudaEventRecord(e0, b->stream);
         for (int k = 0; k < n_trial; k++) RET(sweep_eager(b, n_hits, v));
         cudaEventRecord(e1, b->stream);

@@ -146,14 +146,6 @@ QCB_HD void site_coords(const Geom& g, int par, uint32_t h, int c[4]) {
 QCB_HD int lex_of(const Geom& g, const int c[4]) {
     return c[0] + c[1] * g.stride[1] + c[2] * g.stride[2] + c[3] * g.stride[3];
 }
-QCB_HD void lex_coords(const Geom& g, int64_t lex, int c[4]) {
-    c[0] = (int)(lex % g.L[0]);
-    lex /= g.L[0];
-    c[1] = (int)(lex % g.L[1]);
-    lex /= g.L[1];
-    c[2] = (int)(lex % g.L[2]);
-    c[3] = (int)(lex / g.L[2]);
-}
 // lex index of the site one step up / down in direction d from a site with coordinate cd.
 QCB_HD int step_up(const Geom& g, int lex, int cd, int d) {
     return (cd == g.L[d] - 1) ? lex - (g.L[d] - 1) * g.stride[d] : lex + g.stride[d];

@@ -1077,8 +1077,8 @@ __device__ __forceinline__ void flow_link(const Geom& g, const LinkField<R, NE>&
 // Links of a block of the flow kernels.  FP64: the four warps take the four directions of one tile of
 // 32 half-sites of one parity (blockIdx.x = 2 * tile + parity), so that they read the same neighbour
 // links and share them in L1: with one (mu, parity) class of 128 half-sites a block, each link came
-// from L2 for every use (19 links a link, 10 GB a 32^4 stage at 60% of the L2 rate); L1 now serves 31%
-// of the sectors and a stage takes 649-660 against 695 us (24^4: 185 against 190).  FP32 kernels, bound
+// from L2 for every use (19 links a link, 10 GB a 32^4 stage at 60% of the L2 rate); L1 now serves 29%
+// of the sectors and a stage takes, with the nine-real exponential, 642 against 682 us (24^4: 180 against 191).  FP32 kernels, bound
 // by issue, keep one class a block (blockIdx.x = 8 * site block + mu * 2 + parity): the direction is
 // then uniform over the block (16^4: 30.6 against 31.6 us).
 static_assert(QCB_FLOW_THREADS == 128, "flow_map: four warps a block, and the work lists' tiles of 128 half-sites");

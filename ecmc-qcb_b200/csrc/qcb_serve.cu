@@ -206,7 +206,7 @@ bool grow(qcb_server_s* s, T** p, size_t* cap, size_t n) {
 // Submission was most of a request's time: its FP64 links were copied by one thread into freshly mapped
 // memory (84 ms for a 24^4 configuration) and uploaded in full.  The copy now rounds to the server's
 // format, in up to four threads, into buffers that later requests use again: a 24^4 submission takes 6 ms, and
-// eight requests of 8^4 to 24^4 with 50 measured steps 52 ms instead of 171 (a new server's first 65, not 186).
+// eight requests of 8^4 to 24^4 with 50 measured steps 52 ms instead of 172 (a new server's first 57-63, not 177-200).
 // The buffers stay ordinary memory: page-locking them made the steady state 10 ms shorter, but locking
 // 150 MB beside a running scheduler took a new server's first requests up to 0.9 s.
 constexpr size_t kSplitBytes = (size_t)4 << 20;  // input of a submission beyond which threads share it

@@ -49,7 +49,7 @@ __device__ __forceinline__ const LatDesc* lattice_of(const LatDesc* lats, const 
 // ---------------------------------------------------------------- heatbath, one (parity, MU) phase
 // One thread a half-site of the concatenated tiles (TILE half-sites each), so any BLOCK size covers the
 // same work list.  A grid of resident blocks that walked the list in strides was slower: a sweep of 32
-// chains of 8^4 to 24^4 (FP64-12, 64 threads) 1601 against 1516 us at N_hits = 1, 2252 against 2139 at 2.
+// chains of 8^4 to 24^4 (FP64-12, 64 threads) 1604 against 1465 us at N_hits = 1, 2245 against 2065 at 2.
 template <typename R, int NE, int MU, int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB)
     k_hb_tiles(const LatDesc* __restrict__ lats, const int* __restrict__ tile_lat, const LatDesc one, int ntiles,
