@@ -815,7 +815,7 @@ constexpr int kHbGroupLinks = 16, kHbGroupThreads = 128;
 // The line: one block a SM.  One chain would gain beyond it (10^4: 62 against 131 us), but a link takes twice the
 // SM time of k_hb_subsweep, which chains side by side on their own streams pay once they fill the GPU.  With
 // sweeps issued by the host (18 us each) chains below the line never do: 8, 16 and 32 of 8^4 take 152, 308 and
-// 633 us a round, 167, 315 and 643 with one thread a link and plain launches; 8 of 10^4 would take 319
+// 633 us for a sweep of each, 167, 315 and 643 with one thread a link and plain launches; 8 of 10^4 would take 319
 // against 185.  Captured in one graph, 8 of 8^4 are level (130 and 131 us); 16 and 32, which a Batch sweeps better,
 // take 267 and 550 against 158 and 269.  (Eight lanes a link that all ran its updates took 182, 356 and 732.)
 constexpr int64_t kHbGroupMaxVh = 148 * kHbGroupLinks;
